@@ -108,6 +108,13 @@ template <typename EPI, int AEB> struct FwdConeBinnedB {
     forward_cone_binned_kernel_body<EPI, AEB>(a...);
   }
 };
+template <typename EPI, bool VEC, int EB, bool WIDE> struct FwdConeStreamB {
+  static constexpr int kMaxThreads = WIDE ? 512 : 64, kMinBlocks = WIDE ? 2 : 12;
+  static auto kernel() { return forward_cone_stream_kernel<EPI, VEC, EB, WIDE>; }
+  template <typename... A> __device__ static void run(const A &...a) {
+    forward_cone_stream_kernel_body<EPI, VEC, EB>(a...);
+  }
+};
 template <typename EPI> struct FwdParBinnedB {
   static constexpr int kMaxThreads = 1024, kMinBlocks = 1;
   static auto kernel() { return forward_parallel_binned_kernel<EPI>; }

@@ -652,10 +652,73 @@ int binned_occupancy(int nthr, size_t smem) {
   return n;
 }
 
+// The streamed cone forward (cone_stream.cuh): psf and slice tap radius 1.
+template <typename EPI, bool VEC, int EB, bool WIDE>
+int launch_stream_as(const mbir_geometry *g, int v_start, int v_count, const float *values,
+                     long long P, int band, const FwdBins &b, const EPI &epi, cudaStream_t st,
+                     const char *what) {
+  const Geo geo = make_geo(*g);
+  const int nblk = fwd_nblk(g);
+  const size_t smem = stream_smem(band, EB);
+  const int rc_smem = request_smem(forward_cone_stream_kernel<EPI, VEC, EB, WIDE>, smem, "forward");
+  if (rc_smem) return rc_smem;
+  const int nthr = (g->num_det_rows + kStreamRows - 1) / kStreamRows * 32;
+  // Channel blocks per CTA.  A longer run shares the pixels at block edges and
+  // the CTA's start, but leaves fewer CTAs: two blocks where that still makes
+  // 8 waves of 6 CTAs per SM (a subset step's forward at 320 rows and 720
+  // views 947 -> 897 us with two; at 64 rows and 360 views 99 -> 118 us).
+  const int bpc = !EPI::kViewFastest && WIDE &&
+                          (long long)v_count * nblk / 2 >= (long long)device_sms() * 48 ? 2 : 1;
+  const int grps = (nblk + bpc - 1) / bpc;
+  const dim3 grid = EPI::kViewFastest ? dim3(v_count, grps) : dim3(grps, v_count);
+  tpre(st);
+  launchb<FwdConeStreamB<EPI, VEC, EB, WIDE>>(
+      grid, nthr, smem, st, what, geo, v_start, values, (int)P, band, (const ConeFwdRec *)b.recs,
+      (const int *)b.list, (const int *)b.offs, b.touched, nblk, bpc, epi);
+  MBIR_CHECK_LAUNCH(what);
+  return MBIR_OK;
+}
+
+// Whether the streamed kernel takes a projection.  Its footprint form needs
+// slice taps of radius 1, and its two staging buffers the shared memory.
+// Whole volumes always gain (headline 109 -> 79 ms, 256^3 12.2 -> 8.4 ms, 64
+// rows 3.3 -> 2.6 ms, 16 rows 488 -> 400 us).  A subset step's forward, whose
+// tiles hold few pixels, gains with the detector's rows (us per step: 320
+// rows 1194 -> 897, 256 rows 181 -> 139, 128 rows 101 -> 95, 64 rows 60 -> 61
+// and 65 -> 71 with 16-bit weights), and loses where a warp's 64 rows overhang
+// the detector's end by much (160 rows 129 -> 136): there, and up to 64 rows,
+// one row per thread is the better one.
+template <typename EPI> bool use_stream(const mbir_geometry *g, int band) {
+  if (g->bp_psf_radius != 1 || stream_smem(band, 16) > (size_t)device_attrs().smem_optin)
+    return false;
+  if (EPI::kViewFastest) return true;
+  const int R = g->num_det_rows, warps = (R + 31) / 32, wide = (R + 63) / 64 * 2;
+  return R > kStreamRows && 20 * wide <= 23 * warps;
+}
+
+template <typename EPI>
+int launch_stream(const mbir_geometry *g, int v_start, int v_count, const float *values,
+                  long long P, int band, const FwdBins &b, const EPI &epi, cudaStream_t st,
+                  const char *what) {
+  // whole volumes fill batches of 16 (headline 82 -> 78 ms); a subset's tile
+  // holds some 50 to 100 pixels, where 8 measured faster (919 -> 897 us)
+  constexpr int kWideEB = EPI::kViewFastest ? 16 : 8;
+  if (band % 4 != 0 || !is_aligned16(values))
+    return launch_stream_as<EPI, false, 8, true>(g, v_start, v_count, values, P, band, b, epi, st,
+                                                 what);
+  if (g->num_det_rows > 2 * kStreamRows)
+    return launch_stream_as<EPI, true, kWideEB, true>(g, v_start, v_count, values, P, band, b, epi,
+                                                      st, what);
+  return launch_stream_as<EPI, true, 8, false>(g, v_start, v_count, values, P, band, b, epi, st,
+                                               what);
+}
+
 template <typename EPI>
 int launch_binned(const mbir_geometry *g, int v_start, int v_count, const float *values,
                   long long P, int band, const FwdBins &b, const EPI &epi, cudaStream_t st,
                   const char *what) {
+  if (use_stream<EPI>(g, band))
+    return launch_stream(g, v_start, v_count, values, P, band, b, epi, st, what);
   const Geo geo = make_geo(*g);
   const dim3 grid = EPI::kViewFastest ? dim3(v_count, fwd_nblk(g)) : dim3(fwd_nblk(g), v_count);
   const int nthr = cone_rt_threads(g);

@@ -85,12 +85,67 @@ __device__ __forceinline__ float lds_f32(unsigned a) {
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
   return v;
 }
+__device__ __forceinline__ unsigned lds_u32(unsigned a) {
+  unsigned v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void lds_f32x2(unsigned a, float &x, float &y) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(a));
+}
+__device__ __forceinline__ void sts_f32(unsigned a, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void sts_f2x2(unsigned a, unsigned long long x, unsigned long long y) {
+  asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
+}
+// Two consecutive pairs (16-byte aligned).
+__device__ __forceinline__ void lds_f2x2(unsigned a, unsigned long long &x,
+                                         unsigned long long &y) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a));
+}
 __device__ __forceinline__ float4 lds_f32x4(unsigned a) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                : "r"(a));
   return v;
+}
+
+// ── pairs of floats in one instruction ─────────────────────────────────────
+// sm_100 issues an FP32 add, multiply or FMA on two independent values (one
+// 64-bit register pair) as one instruction, each half rounded as the scalar
+// one.  The kernels that are bound by issue slots carry two rows or slices a
+// lane that way.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_pack(float lo, float hi) {
+  f2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ f2 f2_dup(float x) { return f2_pack(x, x); }
+__device__ __forceinline__ void f2_unpack(f2 v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
+  f2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 
 // ── storage types ──────────────────────────────────────────────────────────
@@ -105,6 +160,30 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 }
 template <> __device__ __forceinline__ __half from_f32<__half>(float v) {
   return __float2half_rn(v);
+}
+
+// Loads and stores of stored values as global accesses (the pointers come out
+// of structures, where the compiler would issue generic ones).  The loads are
+// volatile: they stay ahead of the stores that follow them in the program.
+__device__ __forceinline__ float ldg_f32(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+template <typename T> __device__ __forceinline__ float ldg_f32(const T *p) {
+  unsigned short v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(__cvta_generic_to_global(p)));
+  T t;
+  memcpy(&t, &v, 2);
+  return to_f32(t);
+}
+__device__ __forceinline__ void stg(float *p, float v) {
+  asm volatile("st.global.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v) : "memory");
+}
+template <typename T> __device__ __forceinline__ void stg(T *p, T v) {
+  unsigned short u;
+  memcpy(&u, &v, 2);
+  asm volatile("st.global.u16 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "h"(u) : "memory");
 }
 
 // Four consecutive stored values at p (16-byte aligned for FP32, 8-byte for
@@ -122,6 +201,21 @@ __device__ __forceinline__ void load4(const T *p, float (&o)[4]) {
     const T *t = reinterpret_cast<const T *>(&v);
 #pragma unroll
     for (int k = 0; k < 4; ++k) o[k] = to_f32(t[k]);
+  }
+}
+
+// The same as two pairs.
+template <typename T>
+__device__ __forceinline__ void load4p(const T *p, f2 &a, f2 &b) {
+  if constexpr (sizeof(T) == 4) {
+    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(p));
+    a = v.x;
+    b = v.y;
+  } else {
+    float o[4];
+    load4(p, o);
+    a = f2_pack(o[0], o[1]);
+    b = f2_pack(o[2], o[3]);
   }
 }
 
@@ -274,11 +368,14 @@ __device__ __forceinline__ float inv_cos_from_t(float t) {
 // square root: q >= 1 is never subnormal, so the result equals
 // inv_cos_from_t without rsqrtf's subnormal-input handling.  Used where it
 // measured faster (the forward's cylinder staging).
-__device__ __forceinline__ float inv_cos_from_t_ftz(float t) {
-  const float q = fmaf(t, t, 1.f);
+__device__ __forceinline__ float rsqrt_ftz(float q) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
-  return q * r;
+  return r;
+}
+__device__ __forceinline__ float inv_cos_from_t_ftz(float t) {
+  const float q = fmaf(t, t, 1.f);
+  return q * rsqrt_ftz(q);
 }
 
 // 1 / cos(phi) for the voxel at global slice k of a cone (view, pixel):

@@ -33,6 +33,9 @@ namespace mbir {
 
 constexpr int kThreads = 256;
 constexpr int kListCap = 512;  // forward: pixel records per processing round
+constexpr float kRintMagic = 12582912.f;      // 1.5 * 2^23: x + kRintMagic holds rint(x) in
+constexpr unsigned kRintBits = 0x4B400000u;   // its low bits, above this pattern (|x| < 2^22)
+constexpr int kStreamStep = 32; // streamed forward: a lane's second row after its first
 constexpr int kPad = 8;        // cone back: zero rows either side of the column buffer
 
 // Cache hints (no architectural effect; every address passed is in bounds).
@@ -45,7 +48,7 @@ __device__ __forceinline__ void prefetch_l1(const void *p) {
 
 // ── sinogram readers (resident VCR layout) ─────────────────────────────────
 // value(v, c, m) = scale(v) * get(base(v, c) + m)
-// get4(i, o): the four values at i .. i + 3 as one vector access (i a
+// get4(i, o), get4p(i, a, b): the four values at i .. i + 3 as one vector access (i a
 // multiple of 4 and aligned16() true); aligned16() is checked on the host.
 __host__ __device__ inline bool is_aligned16(const void *p) {
   return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
@@ -58,6 +61,7 @@ struct ReadF32 {
   __device__ __forceinline__ float scale(int) const { return 1.f; }
   __device__ __forceinline__ float get(size_t i) const { return __ldg(s + i); }
   __device__ __forceinline__ void get4(size_t i, float (&o)[4]) const { load4(s + i, o); }
+  __device__ __forceinline__ void get4p(size_t i, f2 &a, f2 &b) const { load4p(s + i, a, b); }
   __host__ bool aligned16() const { return is_aligned16(s); }
 };
 
@@ -70,6 +74,7 @@ struct ReadScaled {
   __device__ __forceinline__ float scale(int v) const { return __ldg(es + v); }
   __device__ __forceinline__ float get(size_t i) const { return to_f32(e[i]); }
   __device__ __forceinline__ void get4(size_t i, float (&o)[4]) const { load4(e + i, o); }
+  __device__ __forceinline__ void get4p(size_t i, f2 &a, f2 &b) const { load4p(e + i, a, b); }
   __host__ bool aligned16() const { return is_aligned16(e); }
 };
 
@@ -94,6 +99,13 @@ struct ReadWeighted {
     load4(w + i, wv);
 #pragma unroll
     for (int k = 0; k < 4; ++k) o[k] = __fmul_rn(wv[k], ev[k]);
+  }
+  __device__ __forceinline__ void get4p(size_t i, f2 &a, f2 &b) const {
+    f2 wa, wb;
+    load4p(e + i, a, b);
+    load4p(w + i, wa, wb);
+    a = f2_mul(wa, a);
+    b = f2_mul(wb, b);
   }
   __host__ bool aligned16() const { return is_aligned16(e) && is_aligned16(w); }
 };
@@ -655,6 +667,39 @@ struct StoreSino {
     }
   }
   __device__ __forceinline__ void end(int) {}
+  using Stream = struct StoreSinoStream;
+};
+
+// The epilogues' streamed forms (cone_stream.cuh): put(s, q) hands over
+// channel c0 + s of rows m0 and m0 + kStreamStep, s increasing from -2 to
+// nch - 1; flush() follows every batch of pixels, finish() the last put.
+// Here every channel is stored.
+struct StoreSinoStream {
+  float *p;
+  size_t channel, row;
+  int nch;
+  bool on0, on1;
+  __device__ __forceinline__ StoreSinoStream(StoreSino &epi, int v, int c0, int nch_, int m0) {
+    const bool vcr = epi.layout == MBIR_LAYOUT_VCR;
+    const size_t per_row = vcr ? 1 : (size_t)epi.C;
+    channel = vcr ? (size_t)epi.R : 1;
+    p = epi.out + (size_t)(v - epi.v_base) * epi.C * epi.R + (size_t)c0 * channel +
+        (size_t)m0 * per_row;
+    row = (size_t)kStreamStep * per_row;
+    nch = nch_;
+    on0 = m0 < epi.R;
+    on1 = m0 + kStreamStep < epi.R;
+  }
+  __device__ __forceinline__ void put(int s, f2 q) {
+    if ((unsigned)s >= (unsigned)nch) return;
+    float a, b, *o = p + (size_t)s * channel;
+    f2_unpack(q, a, b);
+    if (on0) o[0] = a;
+    if (on1) o[row] = b;
+  }
+  __device__ __forceinline__ void flush() {}
+  __device__ __forceinline__ void finish(StoreSino &) {}
+  static __device__ __forceinline__ void pad_partials(const StoreSino &, int, int) {}
 };
 
 template <bool CONE, int NT, typename EPI>

@@ -21,7 +21,7 @@
 // update is bit-reproducible run to run.
 #pragma once
 
-#include "projectors.cuh"
+#include "cone_stream.cuh"
 
 namespace mbir {
 
@@ -361,6 +361,9 @@ __device__ __forceinline__ bool last_cta(unsigned int *counter, unsigned int tot
 // ── 3. forward epilogue: line search + Ad store ───────────────────────────
 // The per-view scale is a power of two, so Ad / scale is formed exactly as
 // Ad * (1 / scale).
+template <typename T> struct LineSearchStream;
+template <typename T> struct RefreshStream;
+
 template <typename T>
 struct LineSearchEpi {
   static constexpr bool kViewFastest = false;  // binned grids: channel blocks on x
@@ -496,6 +499,7 @@ struct LineSearchEpi {
       }
     }
   }
+  using Stream = struct LineSearchStream<T>;
   // A tile that no pixel reaches: A delta is zero there and is not stored
   // (the sinogram update skips untouched tiles).
   __device__ __forceinline__ void empty_tile(int, int, int) {}
@@ -506,6 +510,112 @@ struct LineSearchEpi {
       partials[2 * slot] = fl;
       partials[2 * slot + 1] = fq;
     }
+  }
+};
+
+// Streamed: e and w of slots s and s + 1 are in registers (se, sw) when slot s
+// is put, whose put sends out the loads of slot s + 2.  Running pointers: pe,
+// pw at slot s + 2 and pa at slot s, of row m0 (of row 0 where m0 is off the
+// detector, whose cells are neither stored nor counted).  A row's products
+// are summed in FP32 over about kFwdCB channels, then added to the FP64 sums
+// (flush, once per batch of pixels).
+template <typename T>
+struct LineSearchStream {
+  const T *pe, *pw;
+  T *pa;
+  int R, n_e, n_w, sums;  // n_e, n_w: slots of e and of w to load (0: none)
+  bool on0, on1;
+  float scale, inv_scale, wscale;
+  f2 se[2], sw[2], rl, rq;
+  double fl, fq;
+  __device__ __forceinline__ LineSearchStream(LineSearchEpi<T> &epi, int v, int c0, int nch,
+                                              int m0) {
+    epi.begin(v);
+    R = epi.R;
+    scale = epi.scale;
+    inv_scale = epi.inv_scale;
+    wscale = epi.wscale;
+    fl = fq = 0.0;
+    const int m1 = m0 + kStreamStep;
+    const size_t i0 = ((size_t)v * epi.C + c0) * R;
+    on0 = m0 < R;
+    on1 = m1 < R;
+    pe = epi.e + i0 + (on0 ? m0 : 0);
+    pw = epi.w + (epi.w != nullptr ? i0 + (on0 ? m0 : 0) : 0);
+    pa = epi.ad + i0 + (on0 ? m0 : 0) - (ptrdiff_t)2 * R;
+    n_e = epi.with_sums ? nch : 0;
+    n_w = epi.with_sums && epi.w != nullptr ? nch : 0;
+    se[0] = se[1] = sw[0] = sw[1] = rl = rq = 0;
+    sums = 0;
+    // the tile's operands on their way to L2 while it is computed (lane j:
+    // channels j, j + 32, ...)
+    const int lane = threadIdx.x & 31;
+    for (int s = lane; s < n_e; s += 32) {
+      const size_t i = i0 + (size_t)s * R + (m0 - lane);
+      if (m0 - lane < R) prefetch_l2(epi.e + i);
+      if (m1 - lane < R) prefetch_l2(epi.e + i + kStreamStep);
+      if (n_w) {
+        if (m0 - lane < R) prefetch_l2(epi.w + i);
+        if (m1 - lane < R) prefetch_l2(epi.w + i + kStreamStep);
+      }
+    }
+  }
+  __device__ __forceinline__ void put(int s, f2 q) {
+    const f2 e0 = se[0], w0 = sw[0];
+    se[0] = se[1];
+    sw[0] = sw[1];
+    if (s + 2 < n_e) {
+      float b = 0.f;
+      if (on1) b = ldg_f32(pe + kStreamStep);
+      se[1] = f2_pack(ldg_f32(pe), b);
+      pe += R;
+    }
+    if (s + 2 < n_w) {
+      float b = 0.f;
+      if (on1) b = ldg_f32(pw + kStreamStep);
+      sw[1] = f2_pack(ldg_f32(pw), b);
+      pw += R;
+    }
+    if (s >= 0) {  // (s < nch)
+      float a, b;
+      f2_unpack(f2_mul(q, f2_dup(inv_scale)), a, b);
+      const T sa = from_f32<T>(a), sb = from_f32<T>(b);
+      if (on0) stg(pa, sa);
+      if (on1) stg(pa + kStreamStep, sb);
+      const f2 sc = f2_dup(scale);
+      const f2 adv = f2_mul(f2_pack(to_f32(sa), to_f32(sb)), sc);
+      const f2 ev = f2_mul(e0, sc);
+      const f2 wa = n_w ? f2_mul(f2_mul(w0, f2_dup(wscale)), adv) : adv;
+      rl = f2_fma(wa, ev, rl);
+      rq = f2_fma(wa, adv, rq);
+      ++sums;
+    }
+    pa += R;
+  }
+  __device__ __forceinline__ void flush() {
+    if (sums < kFwdCB - 4) return;
+    add_up();
+  }
+  __device__ __forceinline__ void add_up() {
+    float a, b;
+    f2_unpack(rl, a, b);
+    fl += (double)(on0 ? a : 0.f);
+    fl += (double)(on1 ? b : 0.f);
+    f2_unpack(rq, a, b);
+    fq += (double)(on0 ? a : 0.f);
+    fq += (double)(on1 ? b : 0.f);
+    rl = rq = 0;
+    sums = 0;
+  }
+  __device__ __forceinline__ void finish(LineSearchEpi<T> &epi) {
+    add_up();
+    epi.fl = fl;
+    epi.fq = fq;
+  }
+  // One CTA covers several blocks' partial slots: the others hold zero.
+  static __device__ __forceinline__ void pad_partials(const LineSearchEpi<T> &epi, int lo, int hi) {
+    if (!epi.with_sums) return;
+    for (int i = 2 * lo + threadIdx.x; i < 2 * hi; i += blockDim.x) epi.partials[i] = 0.0;
   }
 };
 
@@ -550,6 +660,7 @@ struct RefreshEpi {
         if (m0 + k < R) cell(v, c0 + j, m0 + k, q[k]);
     }
   }
+  using Stream = struct RefreshStream<T>;
   // A tile that no pixel reaches: A x is zero, so e = y / scale there.
   __device__ __forceinline__ void empty_tile(int v, int c0, int ncb) {
     const float inv = 1.f / __ldg(es + v);
@@ -559,6 +670,47 @@ struct RefreshEpi {
     }
   }
   __device__ __forceinline__ void end(int) {}
+};
+
+// Streamed: y two slots ahead, as in LineSearchStream; every channel is stored.
+template <typename T>
+struct RefreshStream {
+  const float *y;
+  T *e;
+  size_t off;
+  int R, nch;
+  bool on0, on1;
+  float inv_scale;
+  f2 sy[2];
+  __device__ __forceinline__ RefreshStream(RefreshEpi<T> &epi, int v, int c0, int nch_, int m0) {
+    epi.begin(v);
+    inv_scale = epi.inv_scale;
+    y = epi.y;
+    e = epi.e;
+    R = epi.R;
+    nch = nch_;
+    off = ((size_t)v * epi.C + c0) * R + m0;
+    on0 = m0 < R;
+    on1 = m0 + kStreamStep < R;
+    sy[0] = sy[1] = 0;
+  }
+  __device__ __forceinline__ void put(int s, f2 q) {
+    const f2 y0 = sy[0];
+    sy[0] = sy[1];
+    if ((unsigned)(s + 2) < (unsigned)nch) {
+      const float *p = y + off + (size_t)(s + 2) * R;
+      sy[1] = f2_pack(on0 ? __ldg(p) : 0.f, on1 ? __ldg(p + kStreamStep) : 0.f);
+    }
+    if ((unsigned)s >= (unsigned)nch) return;
+    T *o = e + off + (size_t)s * R;
+    float a, b;
+    f2_unpack(f2_mul(f2_sub(y0, q), f2_dup(inv_scale)), a, b);
+    if (on0) o[0] = from_f32<T>(a);
+    if (on1) o[kStreamStep] = from_f32<T>(b);
+  }
+  __device__ __forceinline__ void flush() {}
+  __device__ __forceinline__ void finish(RefreshEpi<T> &) {}
+  static __device__ __forceinline__ void pad_partials(const RefreshEpi<T> &, int, int) {}
 };
 
 // ── 4. alpha ─────────────────────────────────────────────────────────────
