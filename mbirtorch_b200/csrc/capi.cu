@@ -680,30 +680,37 @@ int launch_stream_as(const mbir_geometry *g, int v_start, int v_count, const flo
 }
 
 // Whether the streamed kernel takes a projection.  Its footprint form needs
-// slice taps of radius 1, and its two staging buffers the shared memory.
-// Whole volumes always gain (headline 109 -> 79 ms, 256^3 12.2 -> 8.4 ms, 64
-// rows 3.3 -> 2.6 ms, 16 rows 488 -> 400 us).  A subset step's forward, whose
-// tiles hold few pixels, gains with the detector's rows (us per step: 320
-// rows 1194 -> 897, 256 rows 181 -> 139, 128 rows 101 -> 95, 64 rows 60 -> 61
-// and 65 -> 71 with 16-bit weights), and loses where a warp's 64 rows overhang
-// the detector's end by much (160 rows 129 -> 136): there, and up to 64 rows,
-// one row per thread is the better one.
-template <typename EPI> bool use_stream(const mbir_geometry *g, int band) {
+// slice taps of radius 1, and its two staging buffers the shared memory.  It
+// gains with the detector's rows, and loses where a warp's 64 rows overhang
+// the detector's end by much, against one row per thread in warps of 32 rows
+// (forward_cone_binned_kernel).  Whole volumes (its time over the other's, 180
+// views of 140^2 pixels unless stated): 8 rows 0.82, 24 rows 0.92, 40 rows
+// 1.05, 64 rows 0.79 (256^2), 72 rows 1.03, 88 rows 1.02, 128 rows 0.82
+// (128^2), 140 rows 1.02, 160 rows 1.03, 200 rows 0.81, 256 rows 0.69 (256^2),
+// 320 rows 0.72 (512^2).  Cylinders copied slice by slice (`vec` false): 9 rows
+// 0.66, 41 rows 1.29, 64 rows 1.29, 89 rows 1.06, 128 rows 1.02, 141 rows 0.92,
+// 161 rows 0.90, 201 rows 0.80, 256 rows 0.87.  A subset step's forward, whose
+// tiles hold few pixels: 16 rows 1.14, 64 rows 1.01 (1.09 with 16-bit weights),
+// 97 rows 0.96, 128 rows 0.94, 160 rows 1.06, 256 rows 0.77, 320 rows 0.75.
+template <typename EPI> bool use_stream(const mbir_geometry *g, int band, bool vec) {
   if (g->bp_psf_radius != 1 || stream_smem(band, 16) > (size_t)device_attrs().smem_optin)
     return false;
-  if (EPI::kViewFastest) return true;
-  const int R = g->num_det_rows, warps = (R + 31) / 32, wide = (R + 63) / 64 * 2;
-  return R > kStreamRows && 20 * wide <= 23 * warps;
+  const int R = g->num_det_rows;
+  if (R <= 32) return EPI::kViewFastest;
+  if (!vec) return R > 2 * kStreamRows;
+  if (R <= kStreamRows) return EPI::kViewFastest && R >= kStreamRows * 3 / 4;
+  const int warps = (R + 31) / 32, wide = (R + 63) / 64 * 2;
+  return 20 * wide <= 23 * warps;
 }
 
 template <typename EPI>
 int launch_stream(const mbir_geometry *g, int v_start, int v_count, const float *values,
-                  long long P, int band, const FwdBins &b, const EPI &epi, cudaStream_t st,
-                  const char *what) {
+                  long long P, int band, const FwdBins &b, bool vec, const EPI &epi,
+                  cudaStream_t st, const char *what) {
   // whole volumes fill batches of 16 (headline 82 -> 78 ms); a subset's tile
   // holds some 50 to 100 pixels, where 8 measured faster (919 -> 897 us)
   constexpr int kWideEB = EPI::kViewFastest ? 16 : 8;
-  if (band % 4 != 0 || !is_aligned16(values))
+  if (!vec)
     return launch_stream_as<EPI, false, 8, true>(g, v_start, v_count, values, P, band, b, epi, st,
                                                  what);
   if (g->num_det_rows > 2 * kStreamRows)
@@ -717,8 +724,9 @@ template <typename EPI>
 int launch_binned(const mbir_geometry *g, int v_start, int v_count, const float *values,
                   long long P, int band, const FwdBins &b, const EPI &epi, cudaStream_t st,
                   const char *what) {
-  if (use_stream<EPI>(g, band))
-    return launch_stream(g, v_start, v_count, values, P, band, b, epi, st, what);
+  const bool vec = band % 4 == 0 && is_aligned16(values);
+  if (use_stream<EPI>(g, band, vec))
+    return launch_stream(g, v_start, v_count, values, P, band, b, vec, epi, st, what);
   const Geo geo = make_geo(*g);
   const dim3 grid = EPI::kViewFastest ? dim3(v_count, fwd_nblk(g)) : dim3(fwd_nblk(g), v_count);
   const int nthr = cone_rt_threads(g);
