@@ -16,7 +16,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_NAME = "libmbir_b200.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
 SOURCES = ["capi.cu"]
-HEADERS = ["mbir_common.cuh", "projectors.cuh", "cone_stream.cuh", "vcd.cuh", "batch.cuh"]
+HEADERS = ["mbir_common.cuh", "projectors.cuh", "cone_stream.cuh", "back_cone4.cuh", "vcd.cuh", "batch.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -20,6 +20,7 @@
 #include <utility>
 #include <vector>
 
+#include "back_cone4.cuh"
 #include "vcd.cuh"
 
 namespace mbir {
@@ -94,6 +95,13 @@ template <int CP, int SPL, int NT, typename RD, int HBL = 8> struct BackConeB {
   static auto kernel() { return back_cone_kernel<CP, SPL, NT, RD, HBL>; }
   template <typename... A> __device__ static void run(const A &...a) {
     back_cone_kernel_body<CP, SPL, NT, RD, HBL>(a...);
+  }
+};
+template <int CP, int NP, typename RD> struct BackCone4B {
+  static constexpr int kMaxThreads = kThreads, kMinBlocks = NP == 1 ? 5 : 4;
+  static auto kernel() { return back_cone4_kernel<CP, NP, RD>; }
+  template <typename... A> __device__ static void run(const A &...a) {
+    back_cone4_kernel_body<CP, NP, RD>(a...);
   }
 };
 struct ConeBinB {

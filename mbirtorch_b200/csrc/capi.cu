@@ -376,6 +376,34 @@ int back_long_batch(int R) {
   return s6 < s8 ? 6 : 8;
 }
 
+// The cone back projector with vector columns (back_cone4.cuh): psf radius 1,
+// cylinders of more than 32 slices, detectors of a multiple of four rows whose
+// sinogram is 16-byte aligned, and column indices v * C + c within 31 bits.
+// Up to 32 slices a lane would hold half a pair, and back_cone_kernel's one
+// slice a lane stays.
+template <typename RD>
+bool use_back_cone4(const mbir_geometry *g, int v_count, int band, const RD &rd) {
+  return g->geometry == MBIR_CONE && g->psf_radius == 1 && band > 32 &&
+         g->num_det_rows % 4 == 0 && rd.aligned16() &&
+         (long long)v_count * g->num_det_channels < (1LL << 31);
+}
+
+template <int CP, int NP, typename RD>
+int launch_back_cone4(const Geo &geo, const mbir_geometry *g, const float *vp, int v_start,
+                      int v_count, const BackShape &s, const RD &rd, const int64_t *pix,
+                      long long P, int slice_start, int band, float *dst, cudaStream_t st,
+                      const char *what, const ConeFwdRec *recs) {
+  const size_t smem = back4_smem(g->num_det_rows);
+  const int rc = request_smem(back_cone4_kernel<CP, NP, RD>, smem, what);
+  if (rc) return rc;
+  tpre(st);
+  launchb<BackCone4B<CP, NP, RD>>(dim3(s.blocks_x, s.nchunks), kThreads, smem, st, what, geo, vp,
+                                  v_start, v_count, s.vpc, rd, pix, (int)P, slice_start, band,
+                                  s.slice_chunks, dst, recs);
+  MBIR_CHECK_LAUNCH(what);
+  return MBIR_OK;
+}
+
 template <int CP, int SPL, int NT, typename RD, int HBL = 8>
 int launch_back_t(const Geo &geo, const mbir_geometry *g, const float *vp, int v_start,
                   int v_count, const BackShape &s, const RD &rd, const int64_t *pix, long long P,
@@ -418,6 +446,18 @@ int launch_back_spl(const Geo &geo, const mbir_geometry *g, const float *vp, int
                     const char *what, const ConeFwdRec *recs) {
 #define MBIR_BACK(SPLV) \
   launch_back_t<CP, SPLV, NT>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, recs)
+  if constexpr (NT == 3) {
+    if (use_back_cone4(g, v_count, band, rd)) {
+#define MBIR_BACK_C4(NPV)                                                                    \
+  launch_back_cone4<CP, NPV>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, \
+                             dst, st, what, recs)
+      if (s.SPL == 2) return MBIR_BACK_C4(1);
+      if (s.SPL == 4) return MBIR_BACK_C4(2);
+      if (band <= 192) return MBIR_BACK_C4(3);
+      return MBIR_BACK_C4(4);
+#undef MBIR_BACK_C4
+    }
+  }
   if (g->geometry == MBIR_CONE) {
     switch (s.SPL) {
       case 1: return MBIR_BACK(1);
