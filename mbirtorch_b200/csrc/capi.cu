@@ -408,7 +408,7 @@ template <int CP, int SPL, int NT, typename RD, int HBL = 8>
 int launch_back_t(const Geo &geo, const mbir_geometry *g, const float *vp, int v_start,
                   int v_count, const BackShape &s, const RD &rd, const int64_t *pix, long long P,
                   int slice_start, int band, float *dst, cudaStream_t st, const char *what,
-                  const ConeFwdRec *recs) {
+                  const ConeFwdRec *recs, const TapRule &taps) {
   dim3 grid(s.blocks_x, s.nchunks);
   if (g->geometry == MBIR_CONE) {
     auto k = back_cone_kernel<CP, SPL, NT, RD, HBL>;
@@ -418,12 +418,13 @@ int launch_back_t(const Geo &geo, const mbir_geometry *g, const float *vp, int v
     launchb<BackConeB<CP, SPL, NT, RD, HBL>>(grid, kThreads, s.smem, st, what, geo, vp, v_start,
                                              v_count, s.vpc, rd, pix, (int)P, slice_start, band,
                                              s.slice_chunks, dst, recs);
-  } else if (NT == 3 && SPL == 4 && band % 4 == 0 && rd.aligned16() && is_aligned16(dst)) {
+  } else if (NT == 3 && SPL == 4 && band % 4 == 0 && rd.aligned16() && is_aligned16(dst) &&
+             (long long)v_count * g->num_det_channels < (1LL << 31)) {
     // four consecutive slices per lane: the same teams, one 16-byte load per tap
     tpre(st);
 #define MBIR_BACK4(TV)                                                                       \
   launchb<BackParallel4B<CP, TV, RD>>(grid, kThreads, 0, st, what, geo, vp, v_start, v_count, \
-                                      s.vpc, rd, pix, (int)P, band, s.slice_chunks, dst)
+                                      s.vpc, rd, pix, (int)P, band, s.slice_chunks, taps, dst)
     if (s.T == 32) MBIR_BACK4(32);
     else if (s.T == 16) MBIR_BACK4(16);
     else if (s.T == 8) MBIR_BACK4(8);
@@ -443,9 +444,9 @@ template <int CP, int NT, typename RD>
 int launch_back_spl(const Geo &geo, const mbir_geometry *g, const float *vp, int v_start,
                     int v_count, const BackShape &s, const RD &rd, const int64_t *pix,
                     long long P, int slice_start, int band, float *dst, cudaStream_t st,
-                    const char *what, const ConeFwdRec *recs) {
+                    const char *what, const ConeFwdRec *recs, const TapRule &taps) {
 #define MBIR_BACK(SPLV) \
-  launch_back_t<CP, SPLV, NT>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, recs)
+  launch_back_t<CP, SPLV, NT>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, recs, taps)
   if constexpr (NT == 3) {
     if (use_back_cone4(g, v_count, band, rd)) {
 #define MBIR_BACK_C4(NPV)                                                                    \
@@ -467,7 +468,7 @@ int launch_back_spl(const Geo &geo, const mbir_geometry *g, const float *vp, int
         if constexpr (NT == 3) {
           if (back_long_batch(g->num_det_rows) == 6)
             return launch_back_t<CP, 8, NT, RD, 6>(geo, g, vp, v_start, v_count, s, rd, pix, P,
-                                                   slice_start, band, dst, st, what, recs);
+                                                   slice_start, band, dst, st, what, recs, taps);
         }
         return MBIR_BACK(8);
     }
@@ -480,11 +481,13 @@ template <int CP, typename RD>
 int launch_back_nt(const Geo &geo, const mbir_geometry *g, const float *vp, int v_start,
                    int v_count, const BackShape &s, const RD &rd, const int64_t *pix,
                    long long P, int slice_start, int band, float *dst, cudaStream_t st,
-                   const char *what, const ConeFwdRec *recs) {
+                   const char *what, const ConeFwdRec *recs, const TapRule &taps) {
   if (g->psf_radius == 1)
-    return launch_back_spl<CP, 3>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, recs);
-  return launch_back_spl<CP, 0>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, nullptr);
+    return launch_back_spl<CP, 3>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, recs, taps);
+  return launch_back_spl<CP, 0>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, nullptr, taps);
 }
+
+constexpr size_t kFlagBytes = 256;  // of a back projection's workspace: the scan's flag
 
 // Back projection with a given reader into `out` (or chunk partials in
 // `partials` followed by the fixed-order reduction).  `recs` (cone, psf
@@ -495,11 +498,12 @@ template <typename RD>
 int run_back(const mbir_geometry *g, const float *vp, int v_start, int v_count, const RD &rd,
              const int64_t *pix, long long P, int cp, int slice_start, int band, float *out,
              const BackShape &s, float *partials, cudaStream_t st, bool reduce_into_out,
-             const char *what = "back projection", const ConeFwdRec *recs = nullptr) {
+             const TapRule &taps, const char *what = "back projection",
+             const ConeFwdRec *recs = nullptr) {
   const Geo geo = make_geo(*g);
   float *dst = s.nchunks > 1 ? partials : out;
-  int rc = cp == 2 ? launch_back_nt<2>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, nullptr)
-                   : launch_back_nt<1>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, recs);
+  int rc = cp == 2 ? launch_back_nt<2>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, nullptr, taps)
+                   : launch_back_nt<1>(geo, g, vp, v_start, v_count, s, rd, pix, P, slice_start, band, dst, st, what, recs, taps);
   if (rc) return rc;
   if (s.nchunks > 1 && reduce_into_out) {
     const size_t n = (size_t)P * band;
@@ -1015,11 +1019,11 @@ int vcd_subset_t(const mbir_geometry *g, const float *vp, const mbir_vcd_params 
   if (wts) {
     ReadWeighted<T> rd{err, es, wts, wsc, C, R};
     rc = run_back(g, vp, 0, V, rd, pix, Ps, 1, 0, S, w.grad_part, w.bs, w.grad_part, st, false,
-                  "vcd gradient (back projection)", recs);
+                  TapRule{1, nullptr}, "vcd gradient (back projection)", recs);
   } else {
     ReadScaled<T> rd{err, es, C, R};
     rc = run_back(g, vp, 0, V, rd, pix, Ps, 1, 0, S, w.grad_part, w.bs, w.grad_part, st, false,
-                  "vcd gradient (back projection)", recs);
+                  TapRule{1, nullptr}, "vcd gradient (back projection)", recs);
   }
   if (rc) return rc;
   // 2. direction (reduces the chunk slabs in order)
@@ -1372,7 +1376,7 @@ size_t mbir_back_project_workspace_size(const mbir_geometry *geom, int32_t view_
   const BackShape s = back_shape(geom, view_count, num_pixels, band_len, (size_t)1 << 40);
   const size_t sino = align_up((size_t)view_count * geom->num_det_rows * geom->num_det_channels *
                                sizeof(float));
-  return back_partial_bytes(s, num_pixels, band_len) + sino;
+  return back_partial_bytes(s, num_pixels, band_len) + sino + kFlagBytes;
 }
 
 int32_t mbir_back_project(const mbir_geometry *geom, const float *view_params, int32_t view_start,
@@ -1410,22 +1414,37 @@ int32_t mbir_back_project(const mbir_geometry *geom, const float *view_params, i
   if (workspace_bytes < need_sino || (need_sino && !workspace))
     return fail(MBIR_ERR_WORKSPACE, "workspace of %zu bytes < %zu needed for the layout change",
                 workspace_bytes, need_sino);
-  const size_t partial_budget = workspace ? workspace_bytes - need_sino : 0;
+  // The layout change of a large sinogram also looks for infinities and NaNs,
+  // so that the kernels may leave out the taps of zero weight where there are
+  // none (TapRule).  Below 4 M cells (some 10 us of projection) the flag's
+  // reset would cost what it saves; without a layout change nothing looks.
+  const bool scan = need_sino && sino_bytes >= ((size_t)16 << 20) &&
+                    workspace_bytes >= need_sino + kFlagBytes;
+  const size_t flag_bytes = scan ? kFlagBytes : 0;
+  const size_t partial_budget = workspace ? workspace_bytes - need_sino - flag_bytes : 0;
   const BackShape s = back_shape(geom, view_count, num_pixels, band_len, partial_budget);
   char *ws = static_cast<char *>(workspace);
   const float *vcr = sino;
+  TapRule taps{1, nullptr};
   if (sino_layout == MBIR_LAYOUT_VRC) {
     float *t = reinterpret_cast<float *>(ws);
+    int *flag = nullptr;
+    if (scan) {
+      flag = reinterpret_cast<int *>(ws + need_sino);
+      const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), st);
+      if (e != cudaSuccess) return fail(MBIR_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
+      taps = TapRule{0, flag};
+    }
     dim3 grid((C + 31) / 32, (R + 31) / 32, view_count);
     tpre(st);
-    vrc_to_vcr_kernel<float><<<grid, dim3(32, 8), 0, st>>>(R, C, sino, nullptr, t);
+    vrc_to_vcr_kernel<float><<<grid, dim3(32, 8), 0, st>>>(R, C, sino, nullptr, t, flag);
     MBIR_CHECK_LAUNCH("layout change");
     vcr = t;
   }
-  float *partials = reinterpret_cast<float *>(ws ? ws + need_sino : nullptr);
+  float *partials = reinterpret_cast<float *>(ws ? ws + need_sino + flag_bytes : nullptr);
   ReadF32 rd{vcr, C, R};
   return run_back(geom, view_params, view_start, view_count, rd, pixel_indices, num_pixels,
-                  coeff_power, slice_start, band_len, out, s, partials, st, true);
+                  coeff_power, slice_start, band_len, out, s, partials, st, true, taps);
 }
 
 int32_t mbir_sino_convert(int32_t direction, int32_t views, int32_t rows, int32_t channels,
@@ -1456,11 +1475,11 @@ int32_t mbir_sino_convert(int32_t direction, int32_t views, int32_t rows, int32_
     const float *s = static_cast<const float *>(src);
     tpre(st);
     if (dtype == MBIR_F32)
-      vrc_to_vcr_kernel<float><<<grid, dim3(32, 8), 0, st>>>(R, C, s, scale, static_cast<float *>(dst));
+      vrc_to_vcr_kernel<float><<<grid, dim3(32, 8), 0, st>>>(R, C, s, scale, static_cast<float *>(dst), nullptr);
     else if (dtype == MBIR_BF16)
-      vrc_to_vcr_kernel<__nv_bfloat16><<<grid, dim3(32, 8), 0, st>>>(R, C, s, scale, static_cast<__nv_bfloat16 *>(dst));
+      vrc_to_vcr_kernel<__nv_bfloat16><<<grid, dim3(32, 8), 0, st>>>(R, C, s, scale, static_cast<__nv_bfloat16 *>(dst), nullptr);
     else
-      vrc_to_vcr_kernel<__half><<<grid, dim3(32, 8), 0, st>>>(R, C, s, scale, static_cast<__half *>(dst));
+      vrc_to_vcr_kernel<__half><<<grid, dim3(32, 8), 0, st>>>(R, C, s, scale, static_cast<__half *>(dst), nullptr);
     MBIR_CHECK_LAUNCH("sinogram conversion");
   } else if (direction == 1) {
     dim3 grid((R + 31) / 32, (C + 31) / 32, views);

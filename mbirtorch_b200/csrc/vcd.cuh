@@ -1207,10 +1207,12 @@ view_scale_kernel(int RC, const float *__restrict__ src, float target, float *__
   }
 }
 
-// Tiled transpose per view: f32 (R, C) <-> T (C, R) with scale.
+// Tiled transpose per view: f32 (R, C) <-> T (C, R) with scale.  With
+// `nonfinite`, an infinity or a NaN in the source sets it.
 template <typename T>
 __global__ void vrc_to_vcr_kernel(int R, int C, const float *__restrict__ src,
-                                  const float *__restrict__ scale, T *__restrict__ dst) {
+                                  const float *__restrict__ scale, T *__restrict__ dst,
+                                  int *__restrict__ nonfinite) {
   __shared__ float t[32][33];
   const int v = blockIdx.z;
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -1219,7 +1221,11 @@ __global__ void vrc_to_vcr_kernel(int R, int C, const float *__restrict__ src,
   T *d = dst + (size_t)v * R * C;
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
     const int r = r0 + j, c = c0 + threadIdx.x;
-    if (r < R && c < C) t[j][threadIdx.x] = s[(size_t)r * C + c];
+    if (r < R && c < C) {
+      const float x = s[(size_t)r * C + c];
+      t[j][threadIdx.x] = x;
+      if (nonfinite != nullptr && !isfinite(x)) *nonfinite = 1;
+    }
   }
   __syncthreads();
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
