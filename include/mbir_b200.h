@@ -204,7 +204,8 @@ int32_t mbir_forward_project_binned(const mbir_geometry *geom, const float *view
                                     size_t workspace_bytes, void *stream);
 
 /* Workspace bytes for mbir_forward_project_binned: the bins of
- * min(view_count, views whose records fit 1 GiB) views, at least one; 0 when
+ * min(view_count, views whose records fit 2 GiB, in whole
+ * multiples of the device's SMs) views, at least one; 0 when
  * the geometry is not covered. */
 size_t mbir_forward_project_binned_workspace_size(const mbir_geometry *geom,
                                                   int32_t view_count, int64_t num_pixels);

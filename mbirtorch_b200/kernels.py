@@ -68,7 +68,7 @@ class DeviceProjector:
     radius 1, up to 1024 detector rows): the records of a chunk of views
     are formed and sorted once, and each (view, channel block) CTA walks
     only the pixels that reach it, where the scanning forward tests every
-    pixel in every block.  The workspace (up to about 1 GiB of records, from
+    pixel in every block.  The workspace (up to 2 GiB of records, from
     torch's caching allocator) is the one transient.
     """
 
