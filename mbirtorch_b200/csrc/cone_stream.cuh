@@ -29,7 +29,7 @@
 // level is above 0.57).  One row per thread with the sums in shared memory
 // (forward_cone_binned_kernel) took 1028 M warp instructions for a headline
 // subset step (1602 pixels x 256 slices x 720 views, 320 x 768 detector), this
-// form 696 M; a third of them are the walk, a quarter the epilogue's stores
+// form 723 M; half of them are the walk, a quarter the epilogue's stores
 // and line-search sums.  Measured, CUDA events: that step's forward 1194 ->
 // 897 us; whole volumes 108.8 -> 78.5 ms (headline), 12.2 -> 8.4 ms (256^3,
 // 360 views), 1178 -> 964 us (128^3, 256 views).  Not kept: padding wide
