@@ -204,11 +204,13 @@ __device__ __forceinline__ void load4(const T *p, float (&o)[4]) {
   }
 }
 
-// The same as two pairs.
+// The same as two pairs.  An ordinary (coherent) load: the error sinogram is
+// written by the kernel that its reader may be launched behind
+// (MBIR_PDL_ENTRY), which the read-only path does not allow.
 template <typename T>
 __device__ __forceinline__ void load4p(const T *p, f2 &a, f2 &b) {
   if constexpr (sizeof(T) == 4) {
-    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(p));
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
     a = v.x;
     b = v.y;
   } else {
@@ -217,6 +219,14 @@ __device__ __forceinline__ void load4p(const T *p, f2 &a, f2 &b) {
     a = f2_pack(o[0], o[1]);
     b = f2_pack(o[2], o[3]);
   }
+}
+
+// The same through the read-only path: arrays that nothing writes while the
+// kernel lives.
+__device__ __forceinline__ void load4p_ro(const float *p, f2 &a, f2 &b) {
+  const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(p));
+  a = v.x;
+  b = v.y;
 }
 
 template <typename T>

@@ -61,7 +61,7 @@ struct ReadF32 {
   __device__ __forceinline__ float scale(int) const { return 1.f; }
   __device__ __forceinline__ float get(size_t i) const { return __ldg(s + i); }
   __device__ __forceinline__ void get4(size_t i, float (&o)[4]) const { load4(s + i, o); }
-  __device__ __forceinline__ void get4p(size_t i, f2 &a, f2 &b) const { load4p(s + i, a, b); }
+  __device__ __forceinline__ void get4p(size_t i, f2 &a, f2 &b) const { load4p_ro(s + i, a, b); }
   __host__ bool aligned16() const { return is_aligned16(s); }
 };
 

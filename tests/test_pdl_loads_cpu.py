@@ -1,0 +1,43 @@
+"""The error sinogram is written by the kernel that a VCD gradient is launched
+behind (programmatic dependent launch: the gradient's CTAs may be resident
+while it is).  The read-only path is for memory that no one writes while the
+kernel lives, so no reader of e may use it, in any storage type or width."""
+
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                    'mbirtorch_b200', 'csrc')
+
+
+def _source(name):
+    return re.sub(r'//[^\n]*', '', open(os.path.join(CSRC, name)).read())
+
+
+def _body(src, start):
+    """The brace-delimited block that opens at or after `start`."""
+    a = src.index('{', start)
+    depth = 0
+    for i in range(a, len(src)):
+        depth += {'{': 1, '}': -1}.get(src[i], 0)
+        if depth == 0:
+            return src[a:i + 1]
+    raise AssertionError('unbalanced braces')
+
+
+def test_error_sinogram_readers_use_no_read_only_loads():
+    proj, common = _source('projectors.cuh'), _source('mbir_common.cuh')
+    found = 0
+    for reader in ('ReadScaled', 'ReadWeighted'):
+        body = _body(proj, proj.index(f'struct {reader} {{'))
+        for m in re.finditer(r'void (get\w+)\(|float (get)\(', body):
+            get = _body(body, m.end())
+            assert '__ldg' not in get, (reader, get)
+            for helper in set(re.findall(r'(\w+)\(\s*[ew]\s*\+', get)):
+                defs = [d.end() for d in re.finditer(rf'void {helper}\(', common)]
+                assert defs, helper
+                for d in defs:
+                    code = _body(common, d)
+                    assert '__ldg' not in code and '.nc' not in code, (reader, helper)
+                    found += 1
+    assert found >= 4   # both readers' four-value loads were looked at
