@@ -1,7 +1,7 @@
 // Cone forward projection over the channel-sorted bins, streamed by channel.
 //
-// One CTA owns (view, `bpc` blocks of kFwdCB channels) and walks its run of
-// the sorted list.  Lane l of warp w owns the detector rows 64 w + l and
+// One CTA owns (view, `bpc` blocks of kFwdCB channels, one or two) and walks
+// its run of the sorted list.  Lane l of warp w owns the detector rows 64 w + l and
 // 64 w + l + 32, as the halves of register pairs (f2), so that the work that
 // a warp does once per pixel is shared by 64 rows and most arithmetic is one
 // instruction for both rows.
@@ -92,21 +92,38 @@ __device__ __forceinline__ void forward_cone_stream_kernel_body(
   float *stage = reinterpret_cast<float *>(rec + kStreamCap);
   const bool vf = EPI::kViewFastest;
   const int grp = vf ? blockIdx.y : blockIdx.x, vl = vf ? blockIdx.x : blockIdx.y;
-  const int b0 = grp * bpc, b1 = min(nblk, b0 + bpc);
-  const int c0 = b0 * kFwdCB;
-  const int nch = min(b1 * kFwdCB, g.C) - c0;
+  const int f0 = grp * bpc;  // the CTA's first block
+  int c0 = f0 * kFwdCB;
+  int nch = min(bpc * kFwdCB, g.C - c0);
   const int nkeys = fwd_nkeys(g.C);
   const ConeFwdRec *vrec = recs + (size_t)vl * P;
   const int *vlist = list + (size_t)vl * P;
   const int *voffs = offs + (size_t)vl * (nkeys + 1);
-  const int start = voffs[c0], end = voffs[min(c0 + nch + 2, nkeys)];
+  int start = voffs[c0], end = voffs[min(c0 + nch + 2, nkeys)];
   const int v = v_start + vl;
-  for (int b = b0 + tid; b < b1; b += nthr) touched[(size_t)v * nblk + b] = end > start;
+  if constexpr (!EPI::kViewFastest) {
+    // Of two blocks, one that no pixel reaches is no part of the step: its
+    // cells, which may be dead, are neither read nor counted.
+    if (nch > kFwdCB) {
+      const int second = voffs[c0 + kFwdCB], first_end = voffs[c0 + kFwdCB + 2];
+      if (first_end == start) {
+        start = second;
+        c0 += kFwdCB;
+        nch -= kFwdCB;
+      } else if (second == end) {
+        end = first_end;
+        nch = kFwdCB;
+      }
+    }
+  }
+  for (int b = f0 + tid; b < min(f0 + bpc, nblk); b += nthr)
+    touched[(size_t)v * nblk + b] =
+        end > start && b * kFwdCB >= c0 && b * kFwdCB < c0 + nch;
   if (end == start) {
     epi.empty_tile(v, c0, nch);
     epi.begin(v);
-    epi.end(v * nblk + b0);
-    EPI::Stream::pad_partials(epi, v * nblk + b0 + 1, v * nblk + b1);
+    epi.end(v * nblk + f0);
+    EPI::Stream::pad_partials(epi, v * nblk + f0 + 1, v * nblk + min(f0 + bpc, nblk));
     return;
   }
   // Zeros either side of each staged cylinder (the interiors are written by
@@ -361,8 +378,8 @@ __device__ __forceinline__ void forward_cone_stream_kernel_body(
   }
   advance(nch + 1);
   stream.finish(epi);
-  epi.end(v * nblk + b0);
-  EPI::Stream::pad_partials(epi, v * nblk + b0 + 1, v * nblk + b1);
+  epi.end(v * nblk + f0);
+  EPI::Stream::pad_partials(epi, v * nblk + f0 + 1, v * nblk + min(f0 + bpc, nblk));
 }
 
 // WIDE: detectors of more than kStreamRows * 2 rows (three warps or more a
