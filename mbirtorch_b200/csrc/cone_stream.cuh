@@ -337,8 +337,17 @@ __device__ __forceinline__ void forward_cone_stream_kernel_body(
           add(__float_as_int(jf), w0, w1, w2[u], det[u]);
         }
       };
+      bool crowded = false;
+      if constexpr (!EPI::kViewFastest) {
+        if (nch > kFwdCB)
+          crowded = stream.crowded(
+              (int)lds_u32(rec_s + (unsigned)(nb - 1) * (unsigned)sizeof(StreamRec) + 20u) - cj);
+      }
 #pragma unroll 1
       for (int e4 = 0; e4 < nb; e4 += 4) {
+        if constexpr (!EPI::kViewFastest) {
+          if (crowded) stream.add_up();
+        }
         unsigned four = (todo >> e4) & 15u;
         if (four == 15u && ((fast >> e4) & 15u) == 15u) {  // uniform over the warp
           walk(std::integral_constant<int, 4>{}, {e4, e4 + 1, e4 + 2, e4 + 3});

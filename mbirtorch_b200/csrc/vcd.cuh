@@ -517,8 +517,11 @@ struct LineSearchEpi {
 // is put, whose put sends out the loads of slot s + 2.  Running pointers: pe,
 // pw at slot s + 2 and pa at slot s, of row m0 (of row 0 where m0 is off the
 // detector, whose cells are neither stored nor counted).  A row's products
-// are summed in FP32 over about kFwdCB channels, then added to the FP64 sums
-// (flush, once per batch of pixels).
+// are summed in FP32 over at most kFwdCB channels, as LineSearchEpi::cells
+// does, then added to the FP64 sums: after a batch of pixels (flush), or, in a
+// batch that spans more channels (crowded), after every four pixels, whose
+// channels and the three still open are at most 15; the others between them
+// hold zero.
 template <typename T>
 struct LineSearchStream {
   const T *pe, *pw;
@@ -591,6 +594,9 @@ struct LineSearchStream {
       ++sums;
     }
     pa += R;
+  }
+  __device__ __forceinline__ bool crowded(int channels) const {
+    return sums + channels > kFwdCB;
   }
   __device__ __forceinline__ void flush() {
     if (sums < kFwdCB - 4) return;

@@ -108,3 +108,52 @@ def test_cells_of_a_block_that_no_pixel_reaches_are_not_counted(bad):
     flat2, e2, alpha2 = _step(m, H, None, x0, broken, idx)
     assert alpha2 == alpha and torch.equal(flat2, flat)
     assert torch.equal(e2[:, :, 208:288], e[:, :, 208:288])
+
+
+def test_line_search_sums_at_most_one_block_in_single_precision():
+    """Products so large that a row's sum over one block of 16 channels fits
+    FP32 and over a CTA's two does not, from eight pixels (one batch of the
+    walk) that lie four channels apart."""
+    N, S = 60, 4
+    m = _model(N, S, sigma_y=1.0)
+    m.set_params(no_warning=True, max_alpha=10.0)    # the step's alpha is about 4
+    V = m.get_params('sinogram_shape')[0]
+    prob = _oracle(m, N, S)
+    rows, cols = np.arange(N) * N + N // 2, (N // 2) * N + np.arange(N)
+    one = ovcd.Problem('cone', prob.geom, prob.view_params[:1], (N, N, S), source_iso_dist=4.0 * N)
+
+    def centre(p):
+        a = one.forward(np.ones((1, S)), np.array([p], dtype=np.int64))[0].sum(axis=0)
+        return float(np.sum(a * np.arange(C)) / np.sum(a))
+
+    line = max((rows, cols), key=lambda ps: abs(centre(ps[0]) - centre(ps[-1])))
+    where = np.array([centre(p) for p in line])
+    idx = np.sort([int(line[np.argmin(np.abs(where - ch))]) for ch in range(226, 256, 4)])
+    assert len(set(idx)) == 8
+    idx = np.asarray(idx, dtype=np.int64)
+    # one view carries weight; e = 1000 there, so that products exceed gradients
+    err = np.zeros((V, R, C), dtype=np.float32)
+    err[0] = 1000.0
+    w1 = np.zeros((1, R, C))
+    w1[0] = 1.0
+    H1 = np.ones((N * N, S))
+    H1[idx] = one.back(w1, idx, coeff_power=2)
+    probe = ovcd.SubsetUpdater(one, 1e30 * H1, 1e30 * w1, 1.0, 0.2, max_alpha=10.0,
+                               dc_profile=ovcd.dc_damping_profile(prob))
+    e1 = np.asarray(err[:1], dtype=np.float64)
+    _, oalpha, _ = probe(np.zeros((N * N, S)), e1, idx)
+    Ad = (np.asarray(err[:1], np.float64) - e1)[0] / oalpha       # (R, C)
+    assert 1 < oalpha < 9
+    assert np.abs(Ad[:, :224]).max() == 0 and np.abs(Ad[:, 256:]).max() == 0
+    lin, quad = 1000.0 * Ad, Ad * Ad
+    both = [np.abs(t[:, 224:256].sum(axis=1)).max() for t in (lin, quad)]
+    each = [np.abs(t[:, a:a + 16].sum(axis=1)).max() for t in (lin, quad) for a in (224, 240)]
+    top = float(np.finfo(np.float32).max)
+    W = 1.4 * top / max(both)
+    assert W * max(each) <= 0.8 * top
+    w = torch.zeros((V, R, C), device='cuda')
+    w[0] = W
+    _, _, alpha = _step(m, torch.as_tensor(W * H1, dtype=torch.float32, device='cuda')
+                        .reshape(N, N, S), w, torch.zeros((N * N, S), device='cuda'),
+                        torch.as_tensor(err, device='cuda'), torch.as_tensor(idx, device='cuda'))
+    assert abs(alpha - oalpha) <= 1e-4 * oalpha
