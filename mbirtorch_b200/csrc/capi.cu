@@ -115,11 +115,12 @@ DevAttrs device_attrs() {
 
 inline int device_sms() { return device_attrs().sms; }
 
-// Opt a kernel into `smem` bytes of dynamic shared memory (above the 48 KB
-// default), refusing requests beyond the device's per-block limit.
+// Opt a kernel into `smem` bytes of dynamic shared memory, refusing requests
+// beyond the device's per-block limit.  The 48 KB that need no opting in hold a
+// kernel's static arrays too, of which the largest are 8 KB.
 template <typename K>
 int request_smem(K *k, size_t smem, const char *what) {
-  if (smem <= 48 * 1024) return MBIR_OK;
+  if (smem <= (48 - 8) * 1024) return MBIR_OK;
   const int limit = device_attrs().smem_optin;
   if (smem > (size_t)limit)
     return fail(MBIR_ERR_INVALID, "%s: needs %zu bytes of shared memory per block, above the "
