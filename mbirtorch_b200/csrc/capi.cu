@@ -697,6 +697,16 @@ int binned_occupancy(int nthr, size_t smem) {
   return n;
 }
 
+// Channel blocks per CTA of the streamed cone forward.  A longer run shares
+// the pixels at block edges and the CTA's start, but leaves fewer CTAs: two
+// blocks where that still makes 8 waves of 6 CTAs per SM (a subset step's
+// forward at 320 rows and 720 views 947 -> 897 us with two; at 64 rows and 360
+// views 99 -> 118 us).
+template <typename EPI> int stream_bpc(int v_count, int nblk) {
+  const bool many = (long long)v_count * nblk / 2 >= (long long)device_sms() * 48;
+  return !EPI::kViewFastest && many ? 2 : 1;
+}
+
 // The streamed cone forward (cone_stream.cuh): psf and slice tap radius 1.
 template <typename EPI, bool VEC, int EB, bool WIDE>
 int launch_stream_as(const mbir_geometry *g, int v_start, int v_count, const float *values,
@@ -708,12 +718,7 @@ int launch_stream_as(const mbir_geometry *g, int v_start, int v_count, const flo
   const int rc_smem = request_smem(forward_cone_stream_kernel<EPI, VEC, EB, WIDE>, smem, "forward");
   if (rc_smem) return rc_smem;
   const int nthr = (g->num_det_rows + kStreamRows - 1) / kStreamRows * 32;
-  // Channel blocks per CTA.  A longer run shares the pixels at block edges and
-  // the CTA's start, but leaves fewer CTAs: two blocks where that still makes
-  // 8 waves of 6 CTAs per SM (a subset step's forward at 320 rows and 720
-  // views 947 -> 897 us with two; at 64 rows and 360 views 99 -> 118 us).
-  const int bpc = !EPI::kViewFastest && WIDE &&
-                          (long long)v_count * nblk / 2 >= (long long)device_sms() * 48 ? 2 : 1;
+  const int bpc = WIDE ? stream_bpc<EPI>(v_count, nblk) : 1;
   const int grps = (nblk + bpc - 1) / bpc;
   const dim3 grid = EPI::kViewFastest ? dim3(v_count, grps) : dim3(grps, v_count);
   tpre(st);
@@ -724,45 +729,181 @@ int launch_stream_as(const mbir_geometry *g, int v_start, int v_count, const flo
   return MBIR_OK;
 }
 
-// Whether the streamed kernel takes a projection.  Its footprint form needs
-// slice taps of radius 1, and its two staging buffers the shared memory.  It
-// gains with the detector's rows, and loses where a warp's 64 rows overhang
-// the detector's end by much, against one row per thread in warps of 32 rows
-// (forward_cone_binned_kernel).  Whole volumes (its time over the other's, 180
-// views of 140^2 pixels unless stated): 8 rows 0.82, 24 rows 0.92, 40 rows
-// 1.05, 64 rows 0.79 (256^2), 72 rows 1.03, 88 rows 1.02, 128 rows 0.82
-// (128^2), 140 rows 1.02, 160 rows 1.03, 200 rows 0.81, 256 rows 0.69 (256^2),
-// 320 rows 0.72 (512^2).  Cylinders copied slice by slice (`vec` false): 9 rows
-// 0.66, 41 rows 1.29, 64 rows 1.29, 89 rows 1.06, 128 rows 1.02, 141 rows 0.92,
-// 161 rows 0.90, 201 rows 0.80, 256 rows 0.87.  A subset step's forward, whose
-// tiles hold few pixels: 16 rows 1.14, 64 rows 1.01 (1.09 with 16-bit weights),
-// 97 rows 0.96, 128 rows 0.94, 160 rows 1.06, 256 rows 0.77, 320 rows 0.75.
-template <typename EPI> bool use_stream(const mbir_geometry *g, int band, bool vec) {
+// Pixels that the streamed kernel stages per batch.  A subset's tile holds some
+// 50 to 100 pixels, where 8 measured faster (a headline step's forward 919 ->
+// 897 us).  Whole volumes fill batches of 16 (headline 82 -> 78 ms), and take
+// them on detectors of more than two warps while the two buffers leave three
+// CTAs an SM, or as many as the registers do: 256 slices, 16 pixels against 8:
+// 0.91-0.95 of the time, 512 slices 0.92-1.13, 640 slices 1.06-1.36 (0.96 at
+// 1000 rows, whose CTAs are two either way), 1024 slices 1.12-1.77.
+template <typename EPI> int stream_batch(const mbir_geometry *g, int band, bool vec) {
+  if (!EPI::kViewFastest || !vec || g->num_det_rows <= 2 * kStreamRows) return 8;
+  const int warps = (g->num_det_rows + kStreamRows - 1) / kStreamRows;
+  const size_t per_sm = (size_t)device_attrs().smem_optin + 1024;
+  const int by_smem = (int)(per_sm / (stream_smem(band, 16) + 1024));
+  return by_smem >= std::min(3, 32 / warps) ? 16 : 8;
+}
+
+// CTAs per SM of the streamed kernel (64 registers a thread).
+inline int stream_ctas(const mbir_geometry *g, int band, int eb) {
+  const int warps = (g->num_det_rows + kStreamRows - 1) / kStreamRows;
+  const size_t per_sm = (size_t)device_attrs().smem_optin + 1024;
+  return std::min(32 / warps, (int)(per_sm / (stream_smem(band, eb) + 1024)));
+}
+
+// The one-row-per-thread kernel's staging for a projection, and its CTAs per SM.
+struct BinnedPick {
+  int variant, ctas;
+};
+template <typename EPI> BinnedPick binned_pick(const mbir_geometry *g, int band, bool vec);
+
+// Whether the streamed kernel takes a projection; else one row per thread in
+// warps of 32 rows (forward_cone_binned_kernel).  The streamed form has half
+// the warps, with more to do per pixel batch.  It gains with the rows, with the
+// pixels of a tile (n below) and with CTAs that fill the device, and loses
+// where a warp's 64 rows overhang the detector's end, where a CTA's start and
+// end are most of it, and with the weights' second load per cell.  Cylinders
+// from 512 slices on cost the other kernel its CTAs.  Figures: its time over
+// the other's, 30 to 720 views of 67^2 to 256^2 pixels (16-channel CTAs).
+//
+// Whole cylinders into a sinogram:
+//  up to 32 rows: n = 20 1.00, n = 37 0.92-1.01, n = 75 0.82-1.00 up to 16 CTAs
+//   an SM, 1.02-1.10 beyond; copied slice by slice n = 37 0.95-1.05, n = 75
+//   0.91-1.00 up to 12, 1.05-1.20 beyond; up to 16 slices, two pixels a warp
+//   there, n = 18 0.77-1.00 at any count, n = 11 to 1.06; 511 slices 0.49-0.71;
+//  48 to 64 rows: 1.00-1.47 below 15 CTAs an SM, 0.93-1.02 at 19, 0.83-0.95 at 29
+//   (n = 11 1.00, n = 6 1.07); 512 slices 0.78-0.94; slice by slice 1.03-1.22;
+//  97 to 128 rows: 1.00-1.14 at 2-4 CTAs an SM, 0.84-1.03 at 5-8, 0.77-0.93 from
+//   15 on; 512 slices 0.71-0.92; slice by slice 0.73-1.21;
+//  129 to 160 rows: 1.02 in vector copies (1024 slices 0.6, left as it was);
+//   slice by slice 130 rows 0.83-1.09 up to 10 CTAs an SM, 0.82-0.95 from 15 on,
+//   160 rows 0.87-1.05 up to 5, 0.82-1.00 from 7 on;
+//  161 to 192 rows: 1.00-1.22 at 2-5 CTAs an SM, 0.82-1.00 from 7 on; 512 slices
+//   0.71-0.92 in vector copies, 1.00-1.10 slice by slice at 2-4;
+//  more: 0.73-0.97, 320 rows 0.72 (512^2).
+// A subset step's forward (many: two channel blocks a CTA):
+//  97 to 128 rows: n = 3 1.05-1.09, n = 9 0.96-1.04, n = 19 0.95-1.03; weights in
+//   16 bits 1.02-1.16; 512 slices from n = 9 on 0.89-0.97 (1200 slices 1.08-1.10),
+//   16-bit weights n = 19 0.98;
+//  129 to 160 rows: vector copies 1.06; slice by slice 1.00-1.10, many 0.92-0.98,
+//   with weights 1.01-1.29;
+//  161 to 192 rows: slice by slice 0.80-0.95; vector copies 1.01-1.06, many 0.89,
+//   16 bits 0.77-0.95, with weights 1.01-1.22;
+//  more: 0.70-1.00, cylinders shorter than the detector n = 6 1.02-1.07;
+//  more than 160 rows with weights: many n = 6 0.90-1.01, n = 9 0.88-0.97; from 24
+//   CTAs an SM n = 9 0.99-1.06, n = 14 0.95-1.02; below n = 19 0.90-1.02, on
+//   cylinders shorter than the detector 1.06-1.14.
+template <typename EPI>
+bool use_stream(const mbir_geometry *g, long long P, int band, bool vec, const EPI &epi) {
   if (g->bp_psf_radius != 1 || stream_smem(band, 16) > (size_t)device_attrs().smem_optin)
-    return false;
+    return false;  // (two buffers of 8 reach to 3500 slices: 1.06-1.9 at 2048 and 3000)
   const int R = g->num_det_rows;
-  if (R <= 32) return EPI::kViewFastest;
-  if (!vec) return R > 2 * kStreamRows;
-  if (R <= kStreamRows) return EPI::kViewFastest && R >= kStreamRows * 3 / 4;
-  const int warps = (R + 31) / 32, wide = (R + 63) / 64 * 2;
-  return 20 * wide <= 23 * warps;
+  // (of the geometry's views, not the call's: a scan projected in view chunks
+  // takes one kernel, and so the same bits, however it is cut)
+  const long long ctas = (long long)g->num_views * fwd_nblk(g), sms = device_sms();
+  const long long n = P * (kFwdCB + 2) / g->num_det_channels;  // pixels of a tile
+  const bool lng = band >= 480;
+  bool weights = false;
+  if constexpr (EPI::kViewFastest) {
+    if (R <= 32) {
+      if (lng) return n >= 16;
+      if (!vec && band <= 16) return n >= 16;
+      return vec ? n >= 32 && ctas <= 16 * sms : n >= 64 && ctas <= 12 * sms;
+    }
+    if (R <= kStreamRows) return vec && R >= 48 && n >= 11 && (lng || ctas >= 24 * sms);
+    if (R <= 2 * kStreamRows) {
+      if (!vec || R <= 96 || !(lng || ctas >= 6 * sms)) return false;
+    } else if (R <= 160) {
+      if (vec || ctas < (R <= 144 ? 14 : 7) * sms) return false;
+    } else if (R <= 192) {
+      if (!(vec && lng) && ctas < 7 * sms) return false;
+    }
+  } else {
+    const bool fp32 = EPI::kBytes == 4;
+    weights = epi.reads() == 2;
+    const bool many = stream_bpc<EPI>(g->num_views, fwd_nblk(g)) == 2;
+    if (R <= 96) return false;
+    if (R <= 2 * kStreamRows) {
+      return vec && n >= (lng && fp32 ? 8 : 16) && (fp32 || !weights || lng);
+    } else if (R <= 160) {
+      if (vec || weights || !many) return false;
+    } else {
+      if (R <= 192 && vec && (weights || (fp32 && !many))) return false;
+      if (weights) {
+        if (many ? n < 6 : ctas >= 24 * sms ? n < 12 : n < 16 || band < R) return false;
+      } else if (!many && n < 8 && band < R) {
+        return false;
+      }
+    }
+  }
+  // Long cylinders whose staging leaves few warps, by the rows in flight over
+  // the other kernel's.  Subset steps of 200 to 512 rows: 1 (1200 slices) n = 3
+  // to 37 1.14-1.47, with weights more; 1.5 (896 and 1024 slices) n = 3-9
+  // 0.98-1.12, n = 19-37 0.85-0.98, with weights n = 19 1.02-1.13, n = 37
+  // 0.95-1.02; 2 (1536 slices) 0.73-0.93, with weights n = 3 1.01-1.11, n = 9
+  // 0.92-1.02.
+  const int warps = (R + kStreamRows - 1) / kStreamRows;
+  const int cta = stream_ctas(g, band, stream_batch<EPI>(g, band, vec));
+  if (R > 2 * kStreamRows && cta < std::min(4, 32 / warps)) {
+    const int rows = cta * warps * kStreamRows;
+    const int other = binned_pick<EPI>(g, band, vec).ctas * cone_rt_threads(g);
+    if (other > 0) {
+      if (!EPI::kViewFastest && 5 * rows < 7 * other) return false;
+      if (4 * rows < 7 * other ? n < (weights ? 32 : 12) : weights && n < 9) return false;
+    }
+  }
+  return true;
 }
 
 template <typename EPI>
 int launch_stream(const mbir_geometry *g, int v_start, int v_count, const float *values,
                   long long P, int band, const FwdBins &b, bool vec, const EPI &epi,
                   cudaStream_t st, const char *what) {
-  // whole volumes fill batches of 16 (headline 82 -> 78 ms); a subset's tile
-  // holds some 50 to 100 pixels, where 8 measured faster (919 -> 897 us)
-  constexpr int kWideEB = EPI::kViewFastest ? 16 : 8;
   if (!vec)
     return launch_stream_as<EPI, false, 8, true>(g, v_start, v_count, values, P, band, b, epi, st,
                                                  what);
-  if (g->num_det_rows > 2 * kStreamRows)
-    return launch_stream_as<EPI, true, kWideEB, true>(g, v_start, v_count, values, P, band, b, epi,
-                                                      st, what);
-  return launch_stream_as<EPI, true, 8, false>(g, v_start, v_count, values, P, band, b, epi, st,
-                                               what);
+  if (g->num_det_rows <= 2 * kStreamRows)
+    return launch_stream_as<EPI, true, 8, false>(g, v_start, v_count, values, P, band, b, epi, st,
+                                                 what);
+  if constexpr (EPI::kViewFastest) {
+    if (stream_batch<EPI>(g, band, vec) == 16)
+      return launch_stream_as<EPI, true, 16, true>(g, v_start, v_count, values, P, band, b, epi,
+                                                   st, what);
+  }
+  return launch_stream_as<EPI, true, 8, true>(g, v_start, v_count, values, P, band, b, epi, st,
+                                              what);
+}
+
+// Asynchronous staging copies 16-byte chunks: whole cylinders of a multiple of
+// 4 slices from a 16-byte aligned array (`vec`).  Its second stage buffer can
+// cost a CTA per SM (the 256-row detector of the 256^3 cone workload runs 4
+// CTAs per SM synchronously, 3 with two 16-pixel buffers), so it is taken in
+// 16-pixel batches where that keeps the synchronous staging's CTAs per SM, else
+// in 8-pixel batches where those keep them, else not.  The choice for the last
+// (device, threads, band) is kept per thread and epilogue.
+template <typename EPI> BinnedPick binned_pick(const mbir_geometry *g, int band, bool vec) {
+  static thread_local int last_dev = -1, last_nthr = -1, last_band = -1, last_vec = -1;
+  static thread_local BinnedPick last = {0, 0};
+  const int nthr = cone_rt_threads(g);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev != last_dev || nthr != last_nthr || band != last_band || (int)vec != last_vec) {
+    last = {0, binned_occupancy<EPI, 0>(nthr, cone_rt_smem(g, band))};
+    if (vec) {
+      const int n_16 = binned_occupancy<EPI, kFwdEB>(nthr, cone_binned_async_smem(g, band, kFwdEB));
+      const int n_8 =
+          binned_occupancy<EPI, kFwdEB / 2>(nthr, cone_binned_async_smem(g, band, kFwdEB / 2));
+      if (n_16 > 0 && n_16 >= last.ctas)
+        last = {kFwdEB, n_16};
+      else if (n_8 > 0 && n_8 >= last.ctas)
+        last = {kFwdEB / 2, n_8};
+    }
+    last_dev = dev;
+    last_nthr = nthr;
+    last_band = band;
+    last_vec = vec;
+  }
+  return last;
 }
 
 template <typename EPI>
@@ -770,7 +911,7 @@ int launch_binned(const mbir_geometry *g, int v_start, int v_count, const float 
                   long long P, int band, const FwdBins &b, const EPI &epi, cudaStream_t st,
                   const char *what) {
   const bool vec = band % 4 == 0 && is_aligned16(values);
-  if (use_stream<EPI>(g, band, vec))
+  if (use_stream(g, P, band, vec, epi))
     return launch_stream(g, v_start, v_count, values, P, band, b, vec, epi, st, what);
   const Geo geo = make_geo(*g);
   const dim3 grid = EPI::kViewFastest ? dim3(v_count, fwd_nblk(g)) : dim3(fwd_nblk(g), v_count);
@@ -778,30 +919,7 @@ int launch_binned(const mbir_geometry *g, int v_start, int v_count, const float 
   const size_t smem_s = cone_rt_smem(g, band);
   const size_t smem_16 = cone_binned_async_smem(g, band, kFwdEB);
   const size_t smem_8 = cone_binned_async_smem(g, band, kFwdEB / 2);
-  // Asynchronous staging copies 16-byte chunks: whole cylinders of a
-  // multiple of 4 slices from a 16-byte aligned array.  Its second stage
-  // buffer can cost a CTA per SM (the 256-row detector of the 256^3 cone
-  // workload runs 4 CTAs per SM synchronously, 3 with two 16-pixel
-  // buffers), so it is taken in 16-pixel batches where that keeps the
-  // synchronous staging's CTAs per SM, else in 8-pixel batches where those
-  // keep them, else not.  The choice for the last (device, threads, band)
-  // is kept per thread and epilogue.
-  int variant = 0;
-  if (band >= 4 && band % 4 == 0 && (reinterpret_cast<uintptr_t>(values) & 15) == 0) {
-    static thread_local int last_dev = -1, last_nthr = -1, last_band = -1, last_variant = 0;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev != last_dev || nthr != last_nthr || band != last_band) {
-      const int n_s = binned_occupancy<EPI, 0>(nthr, smem_s);
-      const int n_16 = binned_occupancy<EPI, kFwdEB>(nthr, smem_16);
-      const int n_8 = binned_occupancy<EPI, kFwdEB / 2>(nthr, smem_8);
-      last_variant = (n_16 > 0 && n_16 >= n_s) ? kFwdEB : (n_8 > 0 && n_8 >= n_s) ? kFwdEB / 2 : 0;
-      last_dev = dev;
-      last_nthr = nthr;
-      last_band = band;
-    }
-    variant = last_variant;
-  }
+  const int variant = vec ? binned_pick<EPI>(g, band, vec).variant : 0;
   if (variant == kFwdEB)
     return launch_binned_as<EPI, kFwdEB>(geo, grid, nthr, smem_16, v_start, values, P, band, b,
                                          epi, st, what);

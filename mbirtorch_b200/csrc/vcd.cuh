@@ -367,6 +367,8 @@ template <typename T> struct RefreshStream;
 template <typename T>
 struct LineSearchEpi {
   static constexpr bool kViewFastest = false;  // binned grids: channel blocks on x
+  static constexpr int kBytes = sizeof(T);     // of a stored cell
+  int reads() const { return with_sums ? 1 + (w != nullptr) : 0; }  // cells read per cell stored
   const T *e;
   const float *es;
   const T *w;

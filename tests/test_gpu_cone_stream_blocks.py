@@ -26,7 +26,7 @@ def _views():
     return -(-2 * 48 * sms // blocks) + 1
 
 
-def _model(N, S, storage='float32', sigma_y=0.5):
+def _model(N, S, storage='float32', sigma_y=0.5, R=R):
     V = _views()
     ang = np.linspace(0, 2 * np.pi, V, endpoint=False)
     m = mb.ConeBeamModel((V, R, C), ang, source_detector_dist=8.0 * N, source_iso_dist=4.0 * N)
@@ -39,6 +39,7 @@ def _model(N, S, storage='float32', sigma_y=0.5):
 
 def _oracle(m, N, S):
     g = m._geometry()
+    R = g.num_det_rows
     og = OracleGeometry(num_det_rows=R, num_det_channels=C, num_recon_rows=N, num_recon_cols=N,
                         num_slices=S, delta_det_channel=2.0, delta_det_row=2.0,
                         delta_voxel=g.delta_voxel, delta_voxel_row=g.delta_voxel_row,
@@ -57,11 +58,17 @@ def _step(m, H, w, x0, err, idx):
     return flat, e, float(alpha)
 
 
-@pytest.mark.parametrize('weighted,storage', [(False, 'float32'), (True, 'float32'),
-                                              (True, 'float16'), (False, 'bfloat16')])
-def test_step_matches_oracle(weighted, storage):
-    N, S = 470, 8      # the volume's shadow reaches past both ends of the detector
-    m = _model(N, S, storage)
+@pytest.mark.parametrize('R,S,weighted,storage', [
+    (196, 8, False, 'float32'), (196, 200, True, 'float32'), (196, 8, True, 'float16'),
+    (196, 8, False, 'bfloat16'),
+    # cylinders copied slice by slice, and detectors that the streamed kernel
+    # takes with two blocks a CTA only
+    (140, 9, False, 'float32'), (170, 9, True, 'float32'), (170, 9, True, 'float16'),
+    (176, 8, False, 'float32'),
+])
+def test_step_matches_oracle(R, S, weighted, storage):
+    N = 470 if S < 100 else 120    # 470: the shadow reaches past both ends of the detector
+    m = _model(N, S, storage, R=R)
     V = m.get_params('sinogram_shape')[0]
     gen = torch.Generator(device='cuda').manual_seed(11)
     err = torch.randn((V, R, C), generator=gen, device='cuda')
