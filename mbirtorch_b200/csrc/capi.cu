@@ -1543,15 +1543,18 @@ int32_t mbir_back_project(const mbir_geometry *geom, const float *view_params, i
   if (workspace_bytes < need_sino || (need_sino && !workspace))
     return fail(MBIR_ERR_WORKSPACE, "workspace of %zu bytes < %zu needed for the layout change",
                 workspace_bytes, need_sino);
+  const size_t partial_budget = workspace ? workspace_bytes - need_sino : 0;
+  const BackShape s = back_shape(geom, view_count, num_pixels, band_len, partial_budget);
   // The layout change of a large sinogram also looks for infinities and NaNs,
   // so that the kernels may leave out the taps of zero weight where there are
   // none (TapRule).  Below 4 M cells (some 10 us of projection) the flag's
   // reset would cost what it saves; without a layout change nothing looks.
+  // The flag lies behind the partials where the workspace has room for it: a
+  // caller's smaller workspace keeps its view chunks.
+  const size_t flag_at =
+      need_sino + (s.nchunks > 1 ? (size_t)s.nchunks * num_pixels * band_len * sizeof(float) : 0);
   const bool scan = need_sino && sino_bytes >= ((size_t)16 << 20) &&
-                    workspace_bytes >= need_sino + kFlagBytes;
-  const size_t flag_bytes = scan ? kFlagBytes : 0;
-  const size_t partial_budget = workspace ? workspace_bytes - need_sino - flag_bytes : 0;
-  const BackShape s = back_shape(geom, view_count, num_pixels, band_len, partial_budget);
+                    workspace_bytes >= flag_at + sizeof(int);
   char *ws = static_cast<char *>(workspace);
   const float *vcr = sino;
   TapRule taps{1, nullptr};
@@ -1559,7 +1562,7 @@ int32_t mbir_back_project(const mbir_geometry *geom, const float *view_params, i
     float *t = reinterpret_cast<float *>(ws);
     int *flag = nullptr;
     if (scan) {
-      flag = reinterpret_cast<int *>(ws + need_sino);
+      flag = reinterpret_cast<int *>(ws + flag_at);
       const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), st);
       if (e != cudaSuccess) return fail(MBIR_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
       taps = TapRule{0, flag};
@@ -1570,7 +1573,7 @@ int32_t mbir_back_project(const mbir_geometry *geom, const float *view_params, i
     MBIR_CHECK_LAUNCH("layout change");
     vcr = t;
   }
-  float *partials = reinterpret_cast<float *>(ws ? ws + need_sino + flag_bytes : nullptr);
+  float *partials = reinterpret_cast<float *>(ws ? ws + need_sino : nullptr);
   ReadF32 rd{vcr, C, R};
   return run_back(geom, view_params, view_start, view_count, rd, pixel_indices, num_pixels,
                   coeff_power, slice_start, band_len, out, s, partials, st, true, taps);

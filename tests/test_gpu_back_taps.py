@@ -45,6 +45,31 @@ def test_zero_taps_left_out(kind, pitch, bad):
         assert bool(torch.isfinite(skip).all()) == (bad is None)
 
 
+def _back_into(proj, y, idx, band, ws, ws_bytes):
+    out = torch.empty((idx.numel(), band), device='cuda')
+    _lib.call(y.device, 'mbir_back_project', proj.geom, _lib.ptr(proj.view_params), 0, y.shape[0],
+              _lib.ptr(y), _lib.MBIR_LAYOUT_VRC, _lib.ptr(idx), idx.numel(), 1, 0, band,
+              _lib.ptr(out), _lib.ptr(ws), ws_bytes, _lib.stream_of(y.device))
+    return out
+
+
+@pytest.mark.parametrize('N', [60, 112])
+def test_flag_takes_nothing_from_the_partials(N):
+    """The smallest workspace for all view chunks gives the default's bits."""
+    V, R, C = 66, 128, 520
+    proj, _ = _projector('parallel', V, R, C, N, R, 1.0)
+    idx = torch.arange(0, N * N, 7 if N == 60 else 1, device='cuda')
+    y = torch.rand((V, R, C), device='cuda')
+    sino, part = V * R * C * 4, idx.numel() * R * 4
+    size = int(_lib.query(y.device, 'mbir_back_project_workspace_size', proj.geom, V, idx.numel(),
+                          R))
+    chunks = (size - sino) // part
+    assert chunks > 1 or N == 112
+    exact = sino + chunks * part
+    ws = torch.empty(size, dtype=torch.uint8, device='cuda')
+    assert torch.equal(_back_into(proj, y, idx, R, ws, exact), proj.back(y, idx))
+
+
 def test_workspace_without_room_for_the_flag():
     """A workspace that holds the layout change alone still serves."""
     V, R, C, N = 66, 128, 520, 8
