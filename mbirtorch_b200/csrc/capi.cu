@@ -405,6 +405,14 @@ int launch_back_cone4(const Geo &geo, const mbir_geometry *g, const float *vp, i
   return MBIR_OK;
 }
 
+// Whether a back projection takes the four-slice parallel kernel (the same
+// teams as four slices a lane, one 16-byte load per tap), the one reader of a
+// TapRule.
+bool use_back_parallel4(const mbir_geometry *g, int v_count, int band, int spl, bool aligned) {
+  return g->geometry == MBIR_PARALLEL && g->psf_radius == 1 && spl == 4 && band % 4 == 0 &&
+         aligned && (long long)v_count * g->num_det_channels < (1LL << 31);
+}
+
 template <int CP, int SPL, int NT, typename RD, int HBL = 8>
 int launch_back_t(const Geo &geo, const mbir_geometry *g, const float *vp, int v_start,
                   int v_count, const BackShape &s, const RD &rd, const int64_t *pix, long long P,
@@ -419,9 +427,7 @@ int launch_back_t(const Geo &geo, const mbir_geometry *g, const float *vp, int v
     launchb<BackConeB<CP, SPL, NT, RD, HBL>>(grid, kThreads, s.smem, st, what, geo, vp, v_start,
                                              v_count, s.vpc, rd, pix, (int)P, slice_start, band,
                                              s.slice_chunks, dst, recs);
-  } else if (NT == 3 && SPL == 4 && band % 4 == 0 && rd.aligned16() && is_aligned16(dst) &&
-             (long long)v_count * g->num_det_channels < (1LL << 31)) {
-    // four consecutive slices per lane: the same teams, one 16-byte load per tap
+  } else if (use_back_parallel4(g, v_count, band, SPL, rd.aligned16() && is_aligned16(dst))) {
     tpre(st);
 #define MBIR_BACK4(TV)                                                                       \
   launchb<BackParallel4B<CP, TV, RD>>(grid, kThreads, 0, st, what, geo, vp, v_start, v_count, \
@@ -489,6 +495,18 @@ int launch_back_nt(const Geo &geo, const mbir_geometry *g, const float *vp, int 
 }
 
 constexpr size_t kFlagBytes = 256;  // of a back projection's workspace: the scan's flag
+
+// Whether a back projection's layout change looks for infinities and NaNs: the
+// kernel must read the answer, and have enough voxels times views that the taps
+// left out save more than the flag's reset costs, some 4 us.  Time with the
+// scan over that with every tap read, by millions of voxel-views: 9-36 M (200 to
+// 3000 pixels) 1.06-1.12, 46 M 1.03, 92 M 1.00, 146-163 M 0.98, 400 M 0.92-0.94,
+// 4700 M 0.90; short cylinders gain earlier (16 and 32 slices: 36 M 0.90, 73 M
+// 0.89; but 8 M 0.97-1.07).
+bool back_scan(const mbir_geometry *g, int v_count, long long P, int band, const BackShape &s,
+               bool aligned) {
+  return (double)P * v_count * band >= 96e6 && use_back_parallel4(g, v_count, band, s.SPL, aligned);
+}
 
 // Back projection with a given reader into `out` (or chunk partials in
 // `partials` followed by the fixed-order reduction).  `recs` (cone, psf
@@ -1505,7 +1523,8 @@ size_t mbir_back_project_workspace_size(const mbir_geometry *geom, int32_t view_
   const BackShape s = back_shape(geom, view_count, num_pixels, band_len, (size_t)1 << 40);
   const size_t sino = align_up((size_t)view_count * geom->num_det_rows * geom->num_det_channels *
                                sizeof(float));
-  return back_partial_bytes(s, num_pixels, band_len) + sino + kFlagBytes;
+  return back_partial_bytes(s, num_pixels, band_len) + sino +
+         (back_scan(geom, view_count, num_pixels, band_len, s, true) ? kFlagBytes : 0);
 }
 
 int32_t mbir_back_project(const mbir_geometry *geom, const float *view_params, int32_t view_start,
@@ -1545,16 +1564,16 @@ int32_t mbir_back_project(const mbir_geometry *geom, const float *view_params, i
                 workspace_bytes, need_sino);
   const size_t partial_budget = workspace ? workspace_bytes - need_sino : 0;
   const BackShape s = back_shape(geom, view_count, num_pixels, band_len, partial_budget);
-  // The layout change of a large sinogram also looks for infinities and NaNs,
-  // so that the kernels may leave out the taps of zero weight where there are
-  // none (TapRule).  Below 4 M cells (some 10 us of projection) the flag's
-  // reset would cost what it saves; without a layout change nothing looks.
-  // The flag lies behind the partials where the workspace has room for it: a
-  // caller's smaller workspace keeps its view chunks.
+  // The layout change of a large sinogram also looks for infinities and NaNs
+  // where the kernel may leave out the taps of zero weight if there are none
+  // (TapRule; back_scan).  Without a layout change nothing looks.  The flag lies
+  // behind the partials where the workspace has room for it: a caller's smaller
+  // workspace keeps its view chunks.
   const size_t flag_at =
       need_sino + (s.nchunks > 1 ? (size_t)s.nchunks * num_pixels * band_len * sizeof(float) : 0);
-  const bool scan = need_sino && sino_bytes >= ((size_t)16 << 20) &&
-                    workspace_bytes >= flag_at + sizeof(int);
+  const bool scan = need_sino && workspace_bytes >= flag_at + sizeof(int) &&
+                    back_scan(geom, view_count, num_pixels, band_len, s,
+                              is_aligned16(workspace) && (s.nchunks > 1 || is_aligned16(out)));
   char *ws = static_cast<char *>(workspace);
   const float *vcr = sino;
   TapRule taps{1, nullptr};

@@ -1,5 +1,7 @@
 """Back projectors that leave out the channel taps of zero weight: the same
-bits as with every tap read, and infinities and NaNs reach the same voxels."""
+bits as with every tap read, and infinities and NaNs reach the same voxels.
+The layout change looks for those only where the kernel reads the answer, and
+takes no workspace from the partial sums."""
 
 import numpy as np
 import pytest
@@ -29,7 +31,10 @@ def _projector(kind, V, R, C, N, S, pitch):
 @pytest.mark.parametrize('pitch', [1.0, 0.72])   # footprints of two cells; of two or three
 @pytest.mark.parametrize('bad', [None, float('inf'), float('nan')])
 def test_zero_taps_left_out(kind, pitch, bad):
-    V, R, C, N = 66, 128, 520, 20     # above the 4 M cells from which a scan pays
+    """Parallel beam leaves them out from 96 M voxel-views on; cone beam reads
+    every tap in either layout, and checks the layouts against each other."""
+    V, R, C, N = 66, 128, 520, 112
+    assert N * N * V * R >= 96e6
     proj, _ = _projector(kind, V, R, C, N, R, pitch)
     gen = torch.Generator(device='cuda').manual_seed(3)
     y = torch.randn((V, R, C), generator=gen, device='cuda')
@@ -53,7 +58,27 @@ def _back_into(proj, y, idx, band, ws, ws_bytes):
     return out
 
 
-@pytest.mark.parametrize('N', [60, 112])
+@pytest.mark.parametrize('kind,N', [('cone', 60), ('parallel', 60)])
+def test_nothing_scans_where_no_tap_is_left_out(kind, N):
+    """Cone beam, and parallel beam too small to gain: the workspace behind the
+    layout change and the partials is not written (a flag would be)."""
+    V, R, C = 66, 128, 520                      # 4.4 M cells
+    proj, _ = _projector(kind, V, R, C, N, R, 1.0)
+    idx = torch.arange(N * N, device='cuda')
+    y = torch.rand((V, R, C), device='cuda')
+    size = int(_lib.query(y.device, 'mbir_back_project_workspace_size', proj.geom, V, idx.numel(),
+                          R))
+    ws = torch.full((size + 4096,), 0xAB, dtype=torch.uint8, device='cuda')
+    got = _back_into(proj, y, idx, R, ws, size + 4096)
+    assert torch.equal(got, proj.back(y, idx))
+    used = V * R * C * 4
+    part = idx.numel() * R * 4
+    while used + part <= size:                  # whole partial volumes
+        used += part
+    assert bool((ws[used:] == 0xAB).all())
+
+
+@pytest.mark.parametrize('N', [60, 112])        # without and with the scan
 def test_flag_takes_nothing_from_the_partials(N):
     """The smallest workspace for all view chunks gives the default's bits."""
     V, R, C = 66, 128, 520
