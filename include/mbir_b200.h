@@ -204,11 +204,16 @@ int32_t mbir_forward_project_binned(const mbir_geometry *geom, const float *view
                                     size_t workspace_bytes, void *stream);
 
 /* Workspace bytes for mbir_forward_project_binned: the bins of
- * min(view_count, views whose records fit 2 GiB, in whole
+ * min(view_count, views whose records fit 1 GiB, in whole
  * multiples of the device's SMs) views, at least one; 0 when
- * the geometry is not covered. */
+ * the geometry is not covered.  _within: the same for
+ * record_bytes instead of 1 GiB (more is faster for large
+ * volumes, and the same bits). */
 size_t mbir_forward_project_binned_workspace_size(const mbir_geometry *geom,
                                                   int32_t view_count, int64_t num_pixels);
+size_t mbir_forward_project_binned_workspace_size_within(const mbir_geometry *geom,
+                                                         int32_t view_count, int64_t num_pixels,
+                                                         size_t record_bytes);
 
 /* Workspace bytes mbir_back_project needs for this call shape. */
 size_t mbir_back_project_workspace_size(const mbir_geometry *geom,

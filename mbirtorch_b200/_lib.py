@@ -95,6 +95,7 @@ SIGNATURES = {
     "mbir_forward_project_binned": (_i32, [_GP, _vp, _i32, _i32, _vp, _i32, _vp, _i64, _vp,
                                            _i32, _vp, _sz, _vp]),
     "mbir_forward_project_binned_workspace_size": (_sz, [_GP, _i32, _i64]),
+    "mbir_forward_project_binned_workspace_size_within": (_sz, [_GP, _i32, _i64, _sz]),
     "mbir_vcd_refresh_error": (_i32, [_GP, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i32, _vp, _sz,
                                       _vp]),
     "mbir_back_project_workspace_size": (_sz, [_GP, _i32, _i64, _i32]),

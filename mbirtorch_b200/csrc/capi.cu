@@ -1037,12 +1037,14 @@ int run_forward(const mbir_geometry *g, const float *vp, int v_start, int v_coun
 //
 // A view is binned by one CTA, so a chunk of fewer views than the device has
 // SMs leaves some idle, and every chunk ends the forward's grid with a part
-// wave.  The default workspace holds the largest multiple of the SM count whose
-// records fit kFullBinBytes (or what fits, where that is fewer views).  512^2
-// pixels, 720 views in 5 chunks of up to 148 (1.6 GiB) against 8 of 90 in 1
-// GiB: parallel 25.3 + 6.5 -> 22.9 + 5.8 ms (forward + binning), cone 78.3 +
-// 7.3 -> 77.4 + 6.2 ms; 3 chunks of up to 296 views: 22.5 + 5.7 and 76.6 + 5.9.
-constexpr size_t kFullBinBytes = (size_t)2 << 30;  // default record budget
+// wave.  A workspace of a given size holds the largest multiple of the SM count
+// whose records fit it (or what fits, where that is fewer views).  512^2
+// pixels, 720 views in 5 chunks of up to 148 (2 GiB: 1.6 GiB taken) against 8 of
+// 90 in 1 GiB: parallel 25.3 + 6.5 -> 22.9 + 5.8 ms (forward + binning), cone
+// 78.3 + 7.3 -> 77.4 + 6.2 ms; 3 chunks of up to 296 views: 22.5 + 5.7 and 76.6
+// + 5.9.  The default stays at 1 GiB, which is what a caller that budgets its
+// memory by it (the reconstruction server's ledger) is charged.
+constexpr size_t kFullBinBytes = (size_t)1 << 30;  // default record budget
 
 size_t full_bin_bytes(const mbir_geometry *g, long long P, int vc) {
   return align_up((size_t)vc * P * sizeof(ConeFwdRec)) + align_up((size_t)vc * P * sizeof(int)) +
@@ -1404,16 +1406,23 @@ int32_t mbir_forward_project_volume(const mbir_geometry *geom, const float *view
                      geom->num_slices, 0, pixel_indices, epi, st, "forward projection", 1);
 }
 
-size_t mbir_forward_project_binned_workspace_size(const mbir_geometry *geom, int32_t view_count,
-                                                  int64_t num_pixels) {
+size_t mbir_forward_project_binned_workspace_size_within(const mbir_geometry *geom,
+                                                         int32_t view_count, int64_t num_pixels,
+                                                         size_t record_bytes) {
   if (!geom || view_count <= 0 || num_pixels <= 0 || num_pixels >= (1LL << 31)) return 0;
   if (geom->num_views <= 0 || geom->num_det_channels <= 0 || !use_binned(geom)) return 0;
   const size_t per_view = (size_t)num_pixels * (sizeof(ConeFwdRec) + sizeof(int));
   int vc = (int)std::max<size_t>(
-      1, std::min<size_t>((size_t)view_count, kFullBinBytes / std::max<size_t>(per_view, 1)));
+      1, std::min<size_t>((size_t)view_count, record_bytes / std::max<size_t>(per_view, 1)));
   const int sms = device_sms();
   if (vc < view_count && vc > sms) vc = vc / sms * sms;
   return full_bin_bytes(geom, num_pixels, vc);
+}
+
+size_t mbir_forward_project_binned_workspace_size(const mbir_geometry *geom, int32_t view_count,
+                                                  int64_t num_pixels) {
+  return mbir_forward_project_binned_workspace_size_within(geom, view_count, num_pixels,
+                                                           kFullBinBytes);
 }
 
 int32_t mbir_forward_project_binned(const mbir_geometry *geom, const float *view_params,

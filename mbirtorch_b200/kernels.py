@@ -68,11 +68,13 @@ class DeviceProjector:
     radius 1, up to 1024 detector rows): the records of a chunk of views
     are formed and sorted once, and each (view, channel block) CTA walks
     only the pixels that reach it, where the scanning forward tests every
-    pixel in every block.  The workspace (up to 2 GiB of records, from
-    torch's caching allocator) is the one transient.
+    pixel in every block.  The workspace (up to ``bin_bytes`` of records, from
+    torch's caching allocator; 1 GiB where that much is not to be had) is the
+    one transient.
     """
 
     binned_forward = {MBIR_PARALLEL: True, MBIR_CONE: True}
+    bin_bytes = 2 << 30
 
     def __init__(self, geom, view_params, device):
         self.geom = geom
@@ -81,10 +83,22 @@ class DeviceProjector:
         if self.view_params.shape[0] != geom.num_views:
             raise ValueError("view parameter count does not match the geometry's views")
 
-    def _binned_workspace(self, device, view_count, num_pixels):
-        """The binned forward's workspace, or None where it does not apply."""
+    def _binned_workspace(self, device, view_count, num_pixels, lean=False):
+        """The binned forward's workspace, or None where it does not apply.
+        Its size sets how many views are binned at a time, and no bit of the
+        result.  ``lean``: the library's default size, which the server's
+        memory ledger charges."""
         if not self.binned_forward.get(self.geom.geometry, False) or num_pixels <= 0:
             return None
+        if not lean:
+            nbytes = int(_lib.query(device, 'mbir_forward_project_binned_workspace_size_within',
+                                    self.geom, view_count, num_pixels, self.bin_bytes))
+            if nbytes <= 0:
+                return None
+            try:
+                return torch.empty(nbytes, dtype=torch.uint8, device=device)
+            except torch.OutOfMemoryError:
+                pass
         nbytes = int(_lib.query(device, 'mbir_forward_project_binned_workspace_size', self.geom,
                                 view_count, num_pixels))
         if nbytes <= 0:
@@ -124,9 +138,11 @@ class DeviceProjector:
                   stream_of(values.device))
         return out
 
-    def forward_volume(self, flat_volume, pixel_indices, layout=MBIR_LAYOUT_VRC, out=None):
+    def forward_volume(self, flat_volume, pixel_indices, layout=MBIR_LAYOUT_VRC, out=None,
+                       lean=False):
         """Whole cylinders read at rows ``pixel_indices`` of a flat (N*N, S)
-        volume (no gathered copy) -> (V, R, C) [VRC] or (V, C, R) [VCR]."""
+        volume (no gathered copy) -> (V, R, C) [VRC] or (V, C, R) [VCR].
+        ``lean``: within the library's default workspace."""
         g = self.geom
         flat = as_f32_contig(flat_volume)
         idx = as_i64_contig(pixel_indices)
@@ -138,7 +154,7 @@ class DeviceProjector:
                  else (g.num_views, g.num_det_channels, g.num_det_rows))
         if out is None:
             out = torch.empty(shape, dtype=torch.float32, device=flat.device)
-        ws = self._binned_workspace(flat.device, g.num_views, idx.shape[0])
+        ws = self._binned_workspace(flat.device, g.num_views, idx.shape[0], lean)
         if ws is not None:
             self._forward_binned(flat, 1, idx, 0, g.num_views, out, layout, ws)
             return out

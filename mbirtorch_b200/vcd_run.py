@@ -130,7 +130,9 @@ class VcdRun:
             x0 = init_recon
         else:
             log.info('Initializing error sinogram')
-            fwd = m.forward_project(init_recon, output_sharded=True)
+            x = m._recon_device(init_recon)
+            fwd = m.projector.forward_volume(x.reshape(-1, x.shape[-1]), m.full_indices_device(),
+                                             lean=True)
             err_vrc, alpha = error_init(sino, fwd, w_dev, scale)
             del fwd
             # alpha stays on the device: x0 = float32(alpha) * x0, as the
