@@ -21,8 +21,8 @@
 // the psf radius was chosen for) take the clamped trapezoid.
 //
 // What bounds it: the latency of the column loads (they come from L2: 20% of
-// its rate) and the L1 data path (0.85 of its wavefronts); issue slots are
-// 0.58 used.  back_cone_kernel was bound by issue: a headline subset step's
+// its rate) and the L1 data path (0.86 of its wavefronts); issue slots are
+// 0.59 used.  back_cone_kernel was bound by issue: a headline subset step's
 // gradient (1602 pixels x 256 slices x 720 views, 320 rows) took 605 M warp
 // instructions, this form 301 M.  Measured, CUDA events: that gradient 643 ->
 // 468 us, at 256^3 and 360 views 98.6 -> 77.5 us; whole volumes 77.6 -> 52.2 ms

@@ -366,12 +366,14 @@ size_t back_partial_bytes(const BackShape &s, long long P, int band) {
   return s.nchunks > 1 ? align_up((size_t)s.nchunks * P * band * sizeof(float)) : 0;
 }
 
-// Rows per lane of the cone back projector's column batches for bands of
-// more than 64 slices: 6 where 192-row batches cover a column of the
-// detector's R rows in fewer row slots than 256-row ones (R in 257..384, for
-// instance), else 8.  Measured: a 320-row detector's VCD gradient 677 ->
-// 642 us per step with 6; a 256-row detector's 97.8 us with 8 against 103.5
-// with 6.  Every h row is summed the same way at either depth.
+// Rows per lane of back_cone_kernel's column batches for bands of more than
+// 128 slices (on detectors that use_back_cone4 does not take: rows not a
+// multiple of four, or an unaligned sinogram): 6 where 192-row batches cover a
+// column of the detector's R rows in fewer row slots than 256-row ones (R in
+// 257..384, for instance), else 8.  Measured, 6 over 8: 257 to 383 rows 0.85-0.96
+// for whole volumes and 0.89-0.98 for subset gradients of 150, 256 and 300
+// slices; 250 rows 1.05-1.06 at 256 slices.  Every h row is summed the same way
+// at either depth.
 int back_long_batch(int R) {
   const long long s6 = 192LL * ((R + 191) / 192), s8 = 256LL * ((R + 255) / 256);
   return s6 < s8 ? 6 : 8;
@@ -381,7 +383,9 @@ int back_long_batch(int R) {
 // cylinders of more than 32 slices, detectors of a multiple of four rows whose
 // sinogram is 16-byte aligned, and column indices v * C + c within 31 bits.
 // Up to 32 slices a lane would hold half a pair, and back_cone_kernel's one
-// slice a lane stays.
+// slice a lane stays.  Its time over that kernel's, 8 to 4096 rows: 33 to 64
+// slices 0.72-1.00 (2048 rows, 200 pixels 1.13), 65 to 256 slices 0.65-0.90 (60
+// to 200 pixels to 1.00), 260 and 300 slices, two chunks of 256 slots, 0.69-0.90.
 template <typename RD>
 bool use_back_cone4(const mbir_geometry *g, int v_count, int band, const RD &rd) {
   return g->geometry == MBIR_CONE && g->psf_radius == 1 && band > 32 &&
@@ -813,12 +817,13 @@ template <typename EPI> BinnedPick binned_pick(const mbir_geometry *g, int band,
 //   cylinders shorter than the detector 1.06-1.14.
 template <typename EPI>
 bool use_stream(const mbir_geometry *g, long long P, int band, bool vec, const EPI &epi) {
-  if (g->bp_psf_radius != 1 || stream_smem(band, 16) > (size_t)device_attrs().smem_optin)
+  const DevAttrs dev = device_attrs();
+  if (g->bp_psf_radius != 1 || stream_smem(band, 16) > (size_t)dev.smem_optin)
     return false;  // (two buffers of 8 reach to 3500 slices: 1.06-1.9 at 2048 and 3000)
   const int R = g->num_det_rows;
   // (of the geometry's views, not the call's: a scan projected in view chunks
   // takes one kernel, and so the same bits, however it is cut)
-  const long long ctas = (long long)g->num_views * fwd_nblk(g), sms = device_sms();
+  const long long ctas = (long long)g->num_views * fwd_nblk(g), sms = dev.sms;
   const long long n = P * (kFwdCB + 2) / g->num_det_channels;  // pixels of a tile
   const bool lng = band >= 480;
   bool weights = false;

@@ -26,12 +26,12 @@
 // pixel at a time.
 //
 // What bounds it: issue slots (0.67-0.72 of them used; no pipe and no memory
-// level is above 0.57).  One row per thread with the sums in shared memory
+// level is above 0.59).  One row per thread with the sums in shared memory
 // (forward_cone_binned_kernel) took 1028 M warp instructions for a headline
 // subset step (1602 pixels x 256 slices x 720 views, 320 x 768 detector), this
-// form 723 M; half of them are the walk, a quarter the epilogue's stores
+// form 722 M; half of them are the walk, a quarter the epilogue's stores
 // and line-search sums.  Measured, CUDA events: that step's forward 1194 ->
-// 897 us; whole volumes 108.8 -> 78.5 ms (headline), 12.2 -> 8.4 ms (256^3,
+// 896 us; whole volumes 108.8 -> 78.5 ms (headline), 12.2 -> 8.4 ms (256^3,
 // 360 views), 1178 -> 964 us (128^3, 256 views).  Not kept: padding wide
 // enough to leave out the clamps (its shared memory cost CTAs: 64-row
 // detectors 105 -> 178 us), 64-register code for one- and two-warp CTAs (99

@@ -610,12 +610,13 @@ def test_large_subset_step_vs_oracle(slices, subset):
     assert rel_l2(err.cpu().numpy(), oerr) <= 1e-5
 
 
-@pytest.mark.parametrize("rows", [256, 300])
+@pytest.mark.parametrize("rows", [256, 300, 254, 302])
 def test_long_band_back_projection_and_step_vs_oracle(rows):
-    """Cone bands of more than 128 slices (8 slices per lane) on detectors of
-    256 rows (column batches 8 rows deep per lane) and 300 rows (6 rows deep,
-    the depth that covers 257..384 rows in fewer row slots): the sparse back
-    projection and a VCD subset step against the FP64 oracle."""
+    """Cone bands of more than 128 slices on detectors of 256 and 300 rows
+    (vector columns), and where the rows are no multiple of four (8 slices per
+    lane) of 254 rows (column batches 8 rows deep per lane) and 302 rows (6 rows
+    deep, the depth that covers 257..384 rows in fewer row slots): the sparse
+    back projection and a VCD subset step against the FP64 oracle."""
     import oracle
     from oracle import vcd as ovcd
     m = mb.ConeBeamModel((12, rows, 40), np.linspace(0, 2 * np.pi, 12, endpoint=False),
