@@ -521,13 +521,13 @@ def roofline_block(m, torch, y, kt, storage, hbm):
 
 
 # DRAM traffic of one forward + line-search launch of the headline workload's
-# 128-subset step (ncu dram__bytes_read.sum 665.9 MB + dram__bytes_write.sum
-# 518.3 MB, one captured launch): one read of e (439 MB), the A delta store
+# 128-subset step (ncu dram__bytes_read.sum 632.5 MB + dram__bytes_write.sum
+# 499.1 MB, one captured launch): one read of e (439 MB), the A delta store
 # (439 MB) and the records and cylinders.
-TRAFFIC_FWD_LS_FP32 = 1184198848.0
+TRAFFIC_FWD_LS_FP32 = 632496128.0 + 499100416.0
 # Warp instructions of the same launch (ncu smsp__inst_executed.sum), and
-# the SM clock the issue peak is taken at (clocks.max.sm of this pool's B200s).
-WARP_INST_FWD_LS_FP32 = 723406440
+# the SM clock the issue peak is taken at (a B200's clocks.max.sm).
+WARP_INST_FWD_LS_FP32 = 722135074
 SM_MAX_MHZ = 1965
 
 
