@@ -165,7 +165,7 @@ __device__ __forceinline__ void back_cone4_kernel_body(
       int ctr;
       if (CP == 1 && recs != nullptr) {
         // The same values cone_bin_kernel formed for this (view, slot).
-        const ConeFwdRec fr = recs[(size_t)(vg + lane) * P + p];
+        const ConeFwdRec fr = load_rec(recs + (size_t)(vg + lane) * P + p);
         ctr = __float_as_int(fr.c.z);
         w[0] = fr.b.y;
         w[1] = fr.b.z;

@@ -177,6 +177,13 @@ template <typename T> __device__ __forceinline__ float ldg_f32(const T *p) {
   memcpy(&t, &v, 2);
   return to_f32(t);
 }
+__device__ __forceinline__ float4 ldg_f32x4(const float4 *p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
 __device__ __forceinline__ void stg(float *p, float v) {
   asm volatile("st.global.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v) : "memory");
 }

@@ -136,6 +136,16 @@ struct __align__(16) ConeFwdRec {
   float4 c;  // a0, a1 (t(k) = a0 + a1 k), centre channel, value row (int bits)
 };
 
+// A record by ordinary (coherent) loads: a gradient may be launched behind the
+// kernel that forms its records (the tail of the step before, MBIR_PDL_ENTRY).
+__device__ __forceinline__ ConeFwdRec load_rec(const ConeFwdRec *r) {
+  ConeFwdRec v;
+  v.a = ldg_f32x4(&r->a);
+  v.b = ldg_f32x4(&r->b);
+  v.c = ldg_f32x4(&r->c);
+  return v;
+}
+
 // ── back projection: parallel ─────────────────────────────────────────────
 template <int CP, int SPL, int NT, typename RD>
 __device__ __forceinline__ void back_parallel_kernel_body(Geo g, const float *__restrict__ vp, int v_start, int v_count, int vpc,
@@ -496,7 +506,7 @@ __device__ __forceinline__ void back_cone_kernel_body(Geo g, const float *__rest
     __syncwarp();
     if (CP == 1 && MT == 3 && recs != nullptr && lane < nv) {
       // The same values cone_bin_kernel formed for this (view, slot).
-      const ConeFwdRec fr = recs[(size_t)(vg + lane) * P + p];
+      const ConeFwdRec fr = load_rec(recs + (size_t)(vg + lane) * P + p);
       ConeRec r;
       r.ctr = __float_as_int(fr.c.z);
       r.w[0] = fr.b.y;

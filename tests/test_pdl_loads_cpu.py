@@ -1,5 +1,5 @@
-"""The error sinogram is written by the kernel that a VCD gradient is launched
-behind (programmatic dependent launch: the gradient's CTAs may be resident
+"""The error sinogram, and the subset's records, are written by the kernel that
+a VCD gradient is launched behind (programmatic dependent launch: the gradient's CTAs may be resident
 while it is).  The read-only path is for memory that no one writes while the
 kernel lives, so no reader of e may use it, in any storage type or width."""
 
@@ -41,3 +41,18 @@ def test_error_sinogram_readers_use_no_read_only_loads():
                     assert '__ldg' not in code and '.nc' not in code, (reader, helper)
                     found += 1
     assert found >= 4   # both readers' four-value loads were looked at
+
+
+def test_gradient_reads_its_records_by_coherent_loads():
+    """The tail of one step forms the next subset's records, which the gradient
+    behind it reads: through load_rec, whose loads are coherent, and not as an
+    element of the (restrict) parameter, which the compiler may load through
+    the read-only path."""
+    proj, back4, common = (_source(f) for f in ('projectors.cuh', 'back_cone4.cuh',
+                                                'mbir_common.cuh'))
+    for src, kernel in ((proj, 'back_cone_kernel_body('), (back4, 'back_cone4_kernel_body(')):
+        body = _body(src, src.index(kernel))
+        assert 'load_rec(recs' in body and not re.search(r'(?<!load_rec\()\brecs\[', body)
+    assert 'ldg_f32x4' in _body(proj, proj.index('ConeFwdRec load_rec('))
+    asm = _body(common, common.index('float4 ldg_f32x4('))
+    assert 'volatile' in asm and 'ld.global.v4' in asm and '.nc' not in asm
