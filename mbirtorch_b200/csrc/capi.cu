@@ -820,6 +820,8 @@ bool use_stream(const mbir_geometry *g, long long P, int band, bool vec, const E
   const DevAttrs dev = device_attrs();
   if (g->bp_psf_radius != 1 || stream_smem(band, 16) > (size_t)dev.smem_optin)
     return false;  // (two buffers of 8 reach to 3500 slices: 1.06-1.9 at 2048 and 3000)
+  if (cone_rt_smem(g, band) > (size_t)dev.smem_optin && binned_pick<EPI>(g, band, vec).ctas == 0)
+    return true;  // (the other kernel does not fit: 1024 rows and 1580 slices, for instance)
   const int R = g->num_det_rows;
   // (of the geometry's views, not the call's: a scan projected in view chunks
   // takes one kernel, and so the same bits, however it is cut)
